@@ -124,6 +124,9 @@ struct sph_engine {
     bool bins_valid = false;       // B, its packed copies and the cells match A
     bool one_sim = false;          // exactly one live simulation (one_dev)
     int n_cell_sims = 0;           // live simulations on the cell-window passes
+    int n_tile_sims = 0;           // ... of these, on cell tiles
+    int items_max = 0;             // most work items of the cell tiles
+    int *n_items = nullptr;
     bool cl_disabled = false;      // cluster lists did not fit: cell passes only
     SimDev one_dev;
     ClusterSet cl = {};            // tuning.pair_scheme = 1 (sph_cluster.cu)
@@ -334,6 +337,23 @@ void fill_const(SimConst<R> &c, const sph_engine *e, const Sim &S, const SimDev 
     c.kappa = (R)p.thermalk;
 }
 
+// Cell tiles serve simulations whose cells hold at least two particles on
+// average (a block fills its tile once per cell, and a nearly empty cell does
+// not repay it).  The rules are of the simulation alone, so its bits are too.
+bool tile_scheme(int precision, int64_t n, int ncells) {
+    return precision == SPH_FP64 && n >= 2 * (int64_t)ncells;
+}
+// Lanes per particle (log2) of the cell tiles: 32 for a small simulation, which
+// spreads it over more warps, eight otherwise.  Density + force of a step, us,
+// 32 / 16 / 8 lanes: 2D 1,024 particles 94 / 107 / 112, 4,096 230 / 214 / 180;
+// 3D 2,197 particles 571 / 711 / 920, 8,000 1934 / 1691 / 1704.
+int tile_lanes(int64_t n) { return n <= 3072 ? 5 : 3; }
+// Most work items of a simulation.
+int64_t tile_items(int64_t n, int ncells) {
+    const int per = kTileRounds * (32 >> tile_lanes(n));
+    return std::min<int64_t>(n, ncells + n / per);
+}
+
 SimDev make_simdev(const sph_engine *e, const Sim &S) {
     SimDev d;
     memset(&d, 0, sizeof(d));
@@ -353,6 +373,8 @@ SimDev make_simdev(const sph_engine *e, const Sim &S) {
             (a < e->dim && S.win[a] > 0) ? 0.5 * S.edge[a] + 0.5 * d.slack_half[a] : 1e300;
         if (a < e->dim && S.nc[a] == 1) d.small_mask |= (1 << a);
     }
+    d.tile_on = tile_scheme(e->precision, S.n, S.ncells) ? 1 : 0;
+    d.tile_lg = tile_lanes(S.n);
     d.vl_gate2 = S.vl_skin > 0.0 ? 0.0625 * S.vl_skin * S.vl_skin : 1e300;
     d.vl_eskin2 = S.vl_skin > 0.0 ? 0.25 * S.vl_skin * S.vl_skin : 1e300;
     d.active = S.active ? 1 : 0;
@@ -597,6 +619,13 @@ View make_view(const sph_engine *e) {
     View v;
     memset(&v, 0, sizeof(v));
     v.np = e->np_b;
+    v.ncells = e->ncells_total;
+    v.n_tile = e->n_tile_sims;
+    v.n_walk = e->n_cell_sims - e->n_tile_sims;
+    v.n_items = e->n_items;
+    v.item_cell = e->rank;
+    v.item_round = e->cell_of;
+    v.items_max = e->items_max;
     v.persist = e->tune.persistent;
     v.dim = e->dim;
     v.sims = e->sims_d;
@@ -814,9 +843,15 @@ int relayout(sph_engine *e) {
     // marks the simulations that run on cluster pairs (SimDev.cl_on)
     TRY(cluster_setup(e, sd));
     TRY(vl_setup(e));
-    e->n_cell_sims = 0;
+    e->n_cell_sims = e->n_tile_sims = 0;
+    int64_t items = 0;
     for (int s = 0; s < (int)e->sims.size(); ++s)
-        if (e->sims[s].active && !sd[s].cl_on) ++e->n_cell_sims;
+        if (e->sims[s].active && !sd[s].cl_on) {
+            ++e->n_cell_sims;
+            e->n_tile_sims += sd[s].tile_on;
+            if (sd[s].tile_on) items += tile_items(e->sims[s].n, e->sims[s].ncells);
+        }
+    e->items_max = (int)items;
     if (e->one_sim) e->one_dev = sd[last];
     CK(cudaMemcpyAsync(e->sims_d, sd.data(), sizeof(SimDev) * e->cap_s, cudaMemcpyHostToDevice, st));
     CK(cudaStreamSynchronize(st));
@@ -869,7 +904,7 @@ void enqueue_prepare(sph_engine *e, cudaStream_t st, bool gated = false, bool li
         cudaMemsetAsync(e->cell_count, 0, sizeof(int) * std::max(e->ncells_total, 1), st);
     cudaMemsetAsync(e->pair_count, 0, sizeof(unsigned long long) * e->cap_s, st);
     launch_bin(v, e->a_extent, st);
-    launch_scan(e->cell_count, e->cell_start, e->ncells_total, e->scan_tmp, st, gate);
+    launch_scan(e->cell_count, e->cell_start, e->ncells_total, e->scan_tmp, st, gate, e->n_items);
     launch_scatter(v, e->a_extent, st);
     launch_cellsort(v, e->ncells_total, st);
     launch_permute(v, e->precision, st);
@@ -1124,19 +1159,22 @@ int cluster_note_fill(sph_engine *e) {
 }
 
 int64_t kernels_per_step(const sph_engine *e) {
+    // cell windows: a launch for the simulations on tiles and one for the others
+    const int forms = e->n_tile_sims > 0 && e->n_tile_sims < e->n_cell_sims ? 2 : 1;
     if (e->cl.on) {
         // cluster build; per evaluation density, [heat,] force and the stage
         // update; the later evaluations' repacking; the cell-window passes of
         // the other simulations
         int64_t k = kSortKernels + cluster_build_kernels();
         k += (int64_t)e->nstage * (3 + (e->group.heat_flux ? 1 : 0)) + (e->nstage - 1);
-        if (e->n_cell_sims > 0) k += (int64_t)e->nstage * (2 + (e->group.heat_flux ? 1 : 0));
+        if (e->n_cell_sims > 0)
+            k += (int64_t)e->nstage * (2 + (e->group.heat_flux ? 1 : 0)) * forms;
         if (e->any_thermostat) k += 2;
         if (rebin_on_demand(e)) k += 2;
         return k;
     }
     int64_t k = kSortKernels + (e->vl.on ? 1 : 0);   // + the pair lists' build
-    k += (int64_t)e->nstage * (2 + (e->group.heat_flux ? 1 : 0));
+    k += (int64_t)e->nstage * (2 + (e->group.heat_flux ? 1 : 0)) * (e->vl.on ? 1 : forms);
     if (e->any_thermostat) k += 2;
     // collisions: per find 5 kernels + 7 for the levels, one apply per
     // evaluation plus the extra first one, one integrator pass per stage
@@ -1341,6 +1379,7 @@ int alloc_sims(sph_engine *e) {
     TRY(dalloc(&e->err, S));
     TRY(dalloc(&e->err_any, 1));
     TRY(dalloc(&e->rebin_gate, 1));
+    TRY(dalloc(&e->n_items, 1));
     TRY(dalloc(&e->restage_far, 1));
     TRY(dalloc(&e->bin_count, 1));
     CK(cudaMemset(e->rebin_gate, 0, sizeof(int)));
@@ -1362,7 +1401,7 @@ void free_all(sph_engine *e) {
                     e->pk_vel[0], e->pk_vel[1], e->pk_f, e->pk_q, e->pk_fv, e->ue, e->rho, e->rho_l,
                     e->temp, e->pres, e->pco, e->rho0, e->pres0, e->pco0, e->udot, e->f0u,
                     e->acc_u, e->stage_buf, e->sims_d, e->t_scale, e->tsum_part, e->steps_d,
-                    e->pair_count, e->err, e->err_any, e->rebin_gate, e->restage_far,
+                    e->pair_count, e->err, e->err_any, e->rebin_gate, e->restage_far, e->n_items,
                     e->bin_count,
                     e->chunk_sim, e->chunk_start,
                     e->chunk_len, e->cell_xyz};
@@ -2087,11 +2126,12 @@ double kernel_sigma(int kernel, int dim, double h) {
 // particle offset 0): device constants, linear-cell -> Morton map and packed
 // cell coordinates, for callers that provide all device memory themselves.
 // cell_ratio as in sph_tuning; vmax bounds |v| for the cell slack.
-int single_sim_tables(const sph_params *p, int64_t n, double cell_ratio, double vmax,
+int single_sim_tables(const sph_params *p, int precision, int64_t n, double cell_ratio, double vmax,
                       SimDev *dev, std::vector<int> *morton, std::vector<int> *cell_xyz) {
     if (!p || !dev || !morton || !cell_xyz || n <= 0) return SPH_EINVAL;
     sph_engine cfg;
     cfg.group = *p;
+    cfg.precision = precision;
     cfg.dim = p->dim;
     int st = validate_params(&cfg, p);
     if (st != SPH_OK) return st;

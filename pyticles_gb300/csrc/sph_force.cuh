@@ -6,7 +6,7 @@
 //               (integrator.py:14-103), periodic teleport (box.py:33-47) and the
 //               thermostat (particles.py:450-457).
 //
-// Instantiated per precision in sph_force_f32.cu / sph_force_f64.cu.
+// Instantiated per form and dimension in sph_force_*.cu.
 #pragma once
 
 #include "sph_pairs.cuh"
@@ -217,7 +217,7 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
     const T4 *__restrict__ Q = (const T4 *)v.pk_q;
     const int s = v.b_sim[ii];
     const SimDev &S = ONE ? v.one : v.sims[s];
-    if (S.cl_on) return;   // evaluated (and integrated) by the cluster passes
+    if (S.cl_on || (!LIST && S.tile_on)) return;   // cluster passes, cell tiles
     KConst<R> ks = make_kconst<R>(S, 0);
     // the long kernel with pco_i/rho_l,i^2 + pco_j/rho_l,j^2 = -2a folded in
     KConst<R> kl = make_kconst_cohesive<R>(S);
@@ -345,33 +345,35 @@ __global__ void __launch_bounds__(256) k_integrate(View v, int stage, int integ,
     integrate_stage<R, D>(v, S, i, s, stage, integ, vdr, ((const R *)v.udot)[i]);
 }
 
-// the persistent form for the mixed-precision pass only (see density_launch)
-template <typename R, int D, int K, int VH, bool ONE>
+// The forms of the force pass, each instantiated in a translation unit of its
+// own (sph_force_*.cu) per dimension.  The persistent form is for the
+// mixed-precision pass only (see density_launch); FP64 walks serve the
+// simulations that are too sparse for cell tiles.
+enum ForceForm { kForceWalk, kForceList };
+
+template <int FORM, typename R, int D, int K, int VH, bool ONE>
 void force_launch(const View &v, int stage, int mode, int integ, int block, cudaStream_t s) {
-    if constexpr (std::is_same<R, float>::value) {
-        if (v.vl_on) {
-            k_force_vl<D, K, VH, ONE>
-                <<<(v.np + block - 1) / block, block, 0, s>>>(v, stage, mode, integ);
-            return;
-        }
-    }
-    if (std::is_same<R, float>::value && v.persist) {
+    const int grid = (v.np + block - 1) / block;
+    if constexpr (FORM == kForceList) {
+        k_force_vl<D, K, VH, ONE><<<grid, block, 0, s>>>(v, stage, mode, integ);
+    } else if (std::is_same<R, float>::value && v.persist) {
         auto *fn = k_force<R, D, K, VH, ONE, std::is_same<R, float>::value>;
         fn<<<pass_grid(v, fn, block), block, 0, s>>>(v, stage, mode, integ);
     } else {
-        k_force<R, D, K, VH, ONE, false>
-            <<<(v.np + block - 1) / block, block, 0, s>>>(v, stage, mode, integ);
+        k_force<R, D, K, VH, ONE, false><<<grid, block, 0, s>>>(v, stage, mode, integ);
     }
 }
 
-template <typename R>
+template <int FORM, typename R, int D>
 void launch_force_t(const View &v, int kernel, int viscosity, int heat, int integrator, int stage,
                     int mode, int block, cudaStream_t s) {
-    if (v.np <= 0) return;
     const int vh = (viscosity ? 1 : 0) | (heat ? 2 : 0);
-#define SPH_FORCE(VH_)                                                                   \
-    (v.one_sim ? force_launch<R, D, K, VH_, true>(v, stage, mode, integrator, block, s)  \
-               : force_launch<R, D, K, VH_, false>(v, stage, mode, integrator, block, s))
+    // constants from the kernel parameters for a single simulation
+    constexpr bool kOne = std::is_same<R, float>::value;
+#define SPH_FORCE(VH_)                                                                        \
+    (v.one_sim && kOne                                                                        \
+         ? force_launch<FORM, R, D, K, VH_, kOne>(v, stage, mode, integrator, block, s)       \
+         : force_launch<FORM, R, D, K, VH_, false>(v, stage, mode, integrator, block, s))
 #define SPH_FORCE_VH                                                                     \
     switch (vh) {                                                                        \
         case 0: SPH_FORCE(0); break;                                                     \
@@ -379,13 +381,7 @@ void launch_force_t(const View &v, int kernel, int viscosity, int heat, int inte
         case 2: SPH_FORCE(2); break;                                                     \
         default: SPH_FORCE(3); break;                                                    \
     }
-    if (v.dim == 2) {
-        constexpr int D = 2;
-        SPH_DISPATCH_K(kernel, SPH_FORCE_VH);
-    } else {
-        constexpr int D = 3;
-        SPH_DISPATCH_K(kernel, SPH_FORCE_VH);
-    }
+    SPH_DISPATCH_K(kernel, SPH_FORCE_VH);
 #undef SPH_FORCE_VH
 #undef SPH_FORCE
 }

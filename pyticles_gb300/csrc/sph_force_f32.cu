@@ -1,22 +1,36 @@
-// sph_force_f32.cu -- the mixed-precision (FP32 pair arithmetic) force pass and
-// integrator stage, and the precision dispatch of both.
+// sph_force_f32.cu -- the dispatch of the force pass to its forms and the
+// integrator stage pass.
 #include "sph_force.cuh"
 
 namespace sph {
 
-extern template void launch_force_t<double>(const View &, int, int, int, int, int, int, int,
-                                            cudaStream_t);
-extern template void launch_integrate_t<double>(const View &, int, int, cudaStream_t, int);
-template void launch_force_t<float>(const View &, int, int, int, int, int, int, int,
-                                    cudaStream_t);
-template void launch_integrate_t<float>(const View &, int, int, cudaStream_t, int);
+#define SPH_FORM(F, R, D)                                                                     \
+    extern template void launch_force_t<F, R, D>(const View &, int, int, int, int, int, int, \
+                                                 int, cudaStream_t)
+SPH_FORM(kForceWalk, float, 2);
+SPH_FORM(kForceWalk, float, 3);
+SPH_FORM(kForceList, float, 2);
+SPH_FORM(kForceList, float, 3);
+SPH_FORM(kForceWalk, double, 2);
+SPH_FORM(kForceWalk, double, 3);
+#undef SPH_FORM
 
 void launch_force(const View &v, int precision, int kernel, int viscosity, int heat,
                   int integrator, int stage, int mode, int block, cudaStream_t s) {
-    if (precision == SPH_MIXED)
-        launch_force_t<float>(v, kernel, viscosity, heat, integrator, stage, mode, block, s);
-    else
-        launch_force_t<double>(v, kernel, viscosity, heat, integrator, stage, mode, block, s);
+    if (v.np <= 0) return;
+    auto run = [&](auto fn2, auto fn3) {
+        (v.dim == 2 ? fn2 : fn3)(v, kernel, viscosity, heat, integrator, stage, mode, block, s);
+    };
+    if (precision != SPH_MIXED) {
+        if (v.n_tile > 0)
+            tile_force(v, kernel, (viscosity ? 1 : 0) | (heat ? 2 : 0), integrator, stage, mode, s);
+        if (v.n_walk > 0)
+            run(launch_force_t<kForceWalk, double, 2>, launch_force_t<kForceWalk, double, 3>);
+    } else if (v.vl_on) {
+        run(launch_force_t<kForceList, float, 2>, launch_force_t<kForceList, float, 3>);
+    } else {
+        run(launch_force_t<kForceWalk, float, 2>, launch_force_t<kForceWalk, float, 3>);
+    }
 }
 
 void launch_integrate(const View &v, int precision, int integrator, int stage, cudaStream_t s,

@@ -111,6 +111,8 @@ struct SimDev {
     int coll_on;            // hard collisions after each evaluation
     int cl_on;              // the pair passes run on cluster pairs (sph_cluster.cu);
                             // the cell-window passes skip this simulation
+    int tile_on;            // the cell-window passes run by cell tiles (sph_tile.cu)
+    int tile_lg;            // ... with at least 2^tile_lg lanes per particle
     int coll_win[3];        // +-cells searched for collision partners
     double coll_c2;         // collision_cutoff^2 (Force.cutoffsq, forces.py:33)
     SimConst<float> cf;
@@ -120,6 +122,12 @@ struct SimDev {
 // Pointers of the engine buffers (device addresses), passed by value.
 struct View {
     int np;                 // particles in B (sorted, active)
+    int ncells;             // cells of all simulations
+    int n_tile, n_walk;     // simulations on cell tiles / on the per-particle window walk
+    // work items of the cell tiles: a cell and its first round each, listed at
+    // binning (in the sort scratch, free by then); at most items_max
+    int *n_items, *item_cell, *item_round;
+    int items_max;
     int dim;
     SimDev *sims;
     // state A
@@ -187,6 +195,8 @@ struct View {
     float4 *vl_x0;
     SimDev one;
 };
+
+constexpr int kTileRounds = 4;   // rounds of a cell in one item: a warp each
 
 // Strided view of an n x 3 (SoA, stride 1) or n x dim (row-major, stride
 // dim) FP64 array: element (slot, axis a) is p[a][slot * stride].
@@ -328,8 +338,9 @@ void launch_integrate(const View &v, int precision, int integrator, int stage, c
 
 // ---- launch wrappers (sph_sort.cu) ----
 void launch_bin(const View &v, int np_a, cudaStream_t s);
+// (clear: a counter set to 0 on the way, or null)
 void launch_scan(int *count, int *start, int n, int *block_tmp, cudaStream_t s,
-                 const int *gate = nullptr);
+                 const int *gate = nullptr, int *clear = nullptr);
 void launch_scatter(const View &v, int np_a, cudaStream_t s);
 void launch_cellsort(const View &v, int ncells, cudaStream_t s);
 void launch_permute(const View &v, int precision, cudaStream_t s);
@@ -359,6 +370,13 @@ void launch_heat(const View &v, int precision, int kernel, int block, cudaStream
 void launch_force(const View &v, int precision, int kernel, int viscosity, int heat,
                   int integrator, int stage, int mode, int block, cudaStream_t s);
 void launch_tsum(const View &v, int precision, int nsims, cudaStream_t s);
+// The FP64 passes by cell tiles, for the simulations with SimDev.tile_on
+// (sph_tile.cu; vh: bit 0 viscosity, bit 1 heat flux).
+void tile_density(const View &v, int kernel, int stage, cudaStream_t s);
+void tile_heat(const View &v, int kernel, cudaStream_t s);
+void tile_force(const View &v, int kernel, int vh, int integ, int stage, int mode,
+                cudaStream_t s);
+int device_sms();   // SMs of the current device
 void launch_pair_rows(const View &v, int precision, int sim_off, int n, long long *row_count,
                       cudaStream_t s);
 void launch_pair_write(const View &v, int precision, int sim_off, int n,

@@ -21,8 +21,8 @@
 #include "sph_internal.h"
 
 namespace sph {
-int single_sim_tables(const sph_params *p, int64_t n, double cell_ratio, double vmax,
-                      SimDev *dev, std::vector<int> *morton, std::vector<int> *cell_xyz);
+int single_sim_tables(const sph_params *p, int precision, int64_t n, double cell_ratio,
+                      double vmax, SimDev *dev, std::vector<int> *morton, std::vector<int> *cell_xyz);
 }
 
 using namespace sph;
@@ -129,7 +129,7 @@ extern "C" int sph_derivatives_noalloc(const sph_params *p, int32_t precision, i
     const double ratios[] = {0.5, 1.0, 2.0, 4.0};
     int status = SPH_ECAPACITY;
     for (double ratio : ratios) {
-        status = single_sim_tables(p, n, ratio, 0.0, &sd, &morton, &cxyz);
+        status = single_sim_tables(p, precision, n, ratio, 0.0, &sd, &morton, &cxyz);
         if (status != SPH_OK) return status;
         if ((int64_t)morton.size() <= SPH_NOALLOC_MAX_CELLS) break;
         status = SPH_ECAPACITY;
@@ -149,6 +149,9 @@ extern "C" int sph_derivatives_noalloc(const sph_params *p, int32_t precision, i
     View w;
     memset(&w, 0, sizeof(w));
     w.np = (int)n;
+    w.ncells = ncells;
+    w.n_tile = sd.tile_on;
+    w.n_walk = 1 - sd.tile_on;
     w.dim = dim;
     w.sims = c.take<SimDev>(1);
     for (int a = 0; a < 3; ++a) {
@@ -192,6 +195,10 @@ extern "C" int sph_derivatives_noalloc(const sph_params *p, int32_t precision, i
     w.err_any = c.take<int>(1);
     w.t_scale = c.take<double>(1);
     w.steps = c.take<long long>(1);
+    w.n_items = c.take<int>(1);
+    w.item_cell = w.rank;
+    w.item_round = w.cell_of;
+    w.items_max = (int)n;
     if (!c.ok) return SPH_ECAPACITY;
     // the first evaluation reads the sorted state itself
     for (int a = 0; a < 3; ++a) {
@@ -219,7 +226,7 @@ extern "C" int sph_derivatives_noalloc(const sph_params *p, int32_t precision, i
 
     // the engine's passes: counting sort, density, heat, force (no state update)
     launch_bin(w, (int)n, st);
-    launch_scan(w.cell_count, w.cell_start, ncells, scan_tmp, st);
+    launch_scan(w.cell_count, w.cell_start, ncells, scan_tmp, st, nullptr, w.n_items);
     launch_scatter(w, (int)n, st);
     launch_cellsort(w, ncells, st);
     launch_permute(w, precision, st);

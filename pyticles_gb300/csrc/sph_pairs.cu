@@ -27,7 +27,7 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
     const T4 *__restrict__ P = (const T4 *)v.pk_pos_in;
     const int s = v.b_sim[ii];
     const SimDev &S = ONE ? v.one : v.sims[s];
-    if (S.cl_on) return;   // evaluated by the cluster passes
+    if (S.cl_on || (!LIST && S.tile_on)) return;   // cluster passes, cell tiles
     KConst<R> ks = make_kconst<R>(S, 0);
     KConst<R> kl = make_kconst<R>(S, 1);
     BAcc<R> rs, rl;
@@ -53,45 +53,13 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
     {
         PairFrame<R, D> fr;
         fr.init(S);
-        if constexpr (LIST) for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done);
-        else for_pairs<R, D>(v, S, fr, P, i, P[i], body, cell_done);
+        if constexpr (LIST) {
+            for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done);
+        } else {
+            for_pairs<R, D>(v, S, fr, P, i, P[i], body, cell_done);
+        }
     }
-    // EOS in FP64 from the compensated sums plus the FP64 self term
-    // (properties.py:77-78): the temperature T = (u + a rho)/k_B cancels
-    // strongly, so rho enters it with the bits the FP32 sum carried in its
-    // compensation.  p/rho^2 = k_B T / (rho (1 - b rho)); the cohesive factor
-    // pco/rho_l^2 is exactly -a and needs no storage.
-    double rho = S.ws0 + S.sig_s * rs.get64();
-    double rhol = S.wl0 + S.sig_l * rl.get64();
-    double T = (v.ue_in[i] + S.a * rho) * S.inv_kb;
-    if (T < 0.0) T = 0.0;
-    double den = rho * (1.0 - S.b * rho);
-    double fs = S.kb * T * recip64<R>(den);
-    double p = fs * rho * rho;
-    double pco = -S.a * rhol * rhol;
-    R Th = (R)T;
-    ((R *)v.rho)[i] = (R)rho;
-    ((R *)v.rho_l)[i] = (R)rhol;
-    ((R *)v.temp)[i] = Th;
-    ((R *)v.pres)[i] = (R)p;
-    ((R *)v.pco)[i] = (R)pco;
-    if (stage == 0) {
-        ((R *)v.rho0)[i] = (R)rho;
-        ((R *)v.pres0)[i] = (R)p;
-        ((R *)v.pco0)[i] = (R)pco;
-    }
-    // {p/rho^2, rho, T_hi, T_lo}: T as a hi/lo pair so that T_j - T_i in the
-    // heat pass does not lose the low bits
-    ((T4 *)v.pk_f)[i] = make_v4<R>((R)fs, (R)rho, Th, (R)(T - (double)Th));
-    // what the force pass reads of a neighbour, in one 16-byte load in 2D
-    const T4 vi = ((const T4 *)v.pk_vel_in)[i];
-    ((T4 *)v.pk_fv)[i] = D == 2 ? make_v4<R>(vi.x, vi.y, (R)fs, (R)rho)
-                                : make_v4<R>(vi.x, vi.y, vi.z, (R)fs);
-    if (!isfinite((R)p) || !isfinite((R)rho) || !isfinite((R)rhol))
-        set_err(v.err, v.err_any, s, SPH_ENAN);
-    // the pair set of one evaluation: counted at the step's first one only
-    // (the counters are cleared once per step)
-    if (stage == 0) add_pair_count(v.pair_count, s, cnt);
+    density_finish<R, D>(v, S, i, s, stage, rs.get64(), rl.get64(), cnt);
 }
 
 // One thread per particle; PERSIST: the resident blocks of pass_grid walk
@@ -135,7 +103,7 @@ __device__ __forceinline__ void heat_one(const View &v, int i) {
     const T4 *__restrict__ F = (const T4 *)v.pk_f;
     const int s = v.b_sim[ii];
     const SimDev &S = ONE ? v.one : v.sims[s];
-    if (S.cl_on) return;   // evaluated by the cluster passes
+    if (S.cl_on || (!LIST && S.tile_on)) return;   // cluster passes, cell tiles
     KConst<R> ks = make_kconst<R>(S, 0);
     const T4 fi = F[ii];
     BAcc<R> q[3];
@@ -228,18 +196,35 @@ void heat_launch(const View &v, int block, cudaStream_t s) {
 void launch_density(const View &v, int precision, int kernel, int stage, int block,
                     cudaStream_t s) {
     if (v.np <= 0) return;
-    if (v.one_sim)
-        SPH_DISPATCH(precision, v.dim, kernel, (density_launch<R, D, K, true>(v, stage, block, s)));
-    else
-        SPH_DISPATCH(precision, v.dim, kernel, (density_launch<R, D, K, false>(v, stage, block, s)));
+    if (precision == SPH_FP64) {
+        if (v.n_tile > 0) tile_density(v, kernel, stage, s);
+        if (v.n_walk == 0) return;
+    }
+    SPH_DISPATCH(precision, v.dim, kernel, {
+        constexpr bool kOne = std::is_same<R, float>::value;
+        if (v.one_sim && kOne) density_launch<R, D, K, kOne>(v, stage, block, s);
+        else density_launch<R, D, K, false>(v, stage, block, s);
+    });
 }
 
 void launch_heat(const View &v, int precision, int kernel, int block, cudaStream_t s) {
     if (v.np <= 0) return;
-    if (v.one_sim)
-        SPH_DISPATCH(precision, v.dim, kernel, (heat_launch<R, D, K, true>(v, block, s)));
-    else
-        SPH_DISPATCH(precision, v.dim, kernel, (heat_launch<R, D, K, false>(v, block, s)));
+    if (precision == SPH_FP64) {
+        if (v.n_tile > 0) tile_heat(v, kernel, s);
+        if (v.n_walk == 0) return;
+    }
+    SPH_DISPATCH(precision, v.dim, kernel, {
+        constexpr bool kOne = std::is_same<R, float>::value;
+        if (v.one_sim && kOne) heat_launch<R, D, K, kOne>(v, block, s);
+        else heat_launch<R, D, K, false>(v, block, s);
+    });
+}
+
+int device_sms() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 1;
 }
 
 int resident_blocks(const void *kernel, int block) {
@@ -251,10 +236,10 @@ int resident_blocks(const void *kernel, int block) {
     const auto key = std::make_pair(kernel, block * 64 + dev);
     auto it = cache.find(key);
     if (it != cache.end()) return it->second;
-    int sms = 0, per = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int per = 0;
+    const int sms = device_sms();
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, block, 0);
-    const int cap = (sms > 0 ? sms : 1) * (per > 0 ? per : 1);
+    const int cap = sms * (per > 0 ? per : 1);
     cache[key] = cap;
     return cap;
 }

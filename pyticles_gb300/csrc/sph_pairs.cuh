@@ -293,39 +293,77 @@ template <typename F> inline int pass_grid(const View &v, F *kernel, int block) 
 
 // Warp-aggregated per-simulation counter update.
 __device__ __forceinline__ void add_pair_count(unsigned long long *cnt, int s, unsigned c) {
-    unsigned act = __activemask();
-    unsigned grp = __match_any_sync(act, s);
-    unsigned long long tot = 0;
-    // sum over the group (lanes with the same simulation)
-    for (int l = 0; l < 32; ++l) {
-        if (!(act & (1u << l))) continue;
-        unsigned x = __shfl_sync(act, c, l);
-        if (grp & (1u << l)) tot += x;
-    }
-    int leader = __ffs(grp) - 1;
-    if ((threadIdx.x & 31) == leader) atomicAdd(&cnt[s], tot);
+    const unsigned grp = __match_any_sync(__activemask(), s);
+    // a warp's counts sum below 2^32: a particle has fewer than 2^26 neighbours
+    const unsigned tot = __reduce_add_sync(grp, c);
+    if ((threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&cnt[s], (unsigned long long)tot);
 }
 
+// Epilogue of the density passes: the equation of state of particle i from
+// the sums of its pairs' m W / sigma, and the records that the heat and force
+// passes read.
+template <typename R, int D>
+__device__ __forceinline__ void density_finish(const View &v, const SimDev &S, int i, int s,
+                                               int stage, double sum_s, double sum_l,
+                                               unsigned cnt) {
+    using T4 = typename V4<R>::T;
+    // EOS in FP64 from the compensated sums plus the FP64 self term
+    // (properties.py:77-78): the temperature T = (u + a rho)/k_B cancels
+    // strongly, so rho enters it with the bits the FP32 sum carried in its
+    // compensation.  p/rho^2 = k_B T / (rho (1 - b rho)); the cohesive factor
+    // pco/rho_l^2 is exactly -a and needs no storage.
+    double rho = S.ws0 + S.sig_s * sum_s;
+    double rhol = S.wl0 + S.sig_l * sum_l;
+    double T = (v.ue_in[i] + S.a * rho) * S.inv_kb;
+    if (T < 0.0) T = 0.0;
+    double den = rho * (1.0 - S.b * rho);
+    double fs = S.kb * T * recip64<R>(den);
+    double p = fs * rho * rho;
+    double pco = -S.a * rhol * rhol;
+    R Th = (R)T;
+    ((R *)v.rho)[i] = (R)rho;
+    ((R *)v.rho_l)[i] = (R)rhol;
+    ((R *)v.temp)[i] = Th;
+    ((R *)v.pres)[i] = (R)p;
+    ((R *)v.pco)[i] = (R)pco;
+    if (stage == 0) {
+        ((R *)v.rho0)[i] = (R)rho;
+        ((R *)v.pres0)[i] = (R)p;
+        ((R *)v.pco0)[i] = (R)pco;
+    }
+    // {p/rho^2, rho, T_hi, T_lo}: T as a hi/lo pair so that T_j - T_i in the
+    // heat pass does not lose the low bits
+    ((T4 *)v.pk_f)[i] = make_v4<R>((R)fs, (R)rho, Th, (R)(T - (double)Th));
+    // what the force pass reads of a neighbour, in one 16-byte load in 2D
+    const T4 vi = ((const T4 *)v.pk_vel_in)[i];
+    ((T4 *)v.pk_fv)[i] = D == 2 ? make_v4<R>(vi.x, vi.y, (R)fs, (R)rho)
+                                : make_v4<R>(vi.x, vi.y, vi.z, (R)fs);
+    if (!isfinite((R)p) || !isfinite((R)rho) || !isfinite((R)rhol))
+        set_err(v.err, v.err_any, s, SPH_ENAN);
+    // the pair set of one evaluation: counted at the step's first one only
+    // (the counters are cleared once per step)
+    if (stage == 0) add_pair_count(v.pair_count, s, cnt);
+}
 
 // ---- dispatch ----
-#define SPH_DISPATCH(PREC, DIM, KERN, CALL)                                       \
+#define SPH_DISPATCH(PREC, DIM, KERN, ...)                                       \
     do {                                                                          \
         if (PREC == SPH_MIXED) {                                                  \
             using R = float;                                                      \
-            if (DIM == 2) { constexpr int D = 2; SPH_DISPATCH_K(KERN, CALL); }    \
-            else { constexpr int D = 3; SPH_DISPATCH_K(KERN, CALL); }             \
+            if (DIM == 2) { constexpr int D = 2; SPH_DISPATCH_K(KERN, __VA_ARGS__); }    \
+            else { constexpr int D = 3; SPH_DISPATCH_K(KERN, __VA_ARGS__); }             \
         } else {                                                                  \
             using R = double;                                                     \
-            if (DIM == 2) { constexpr int D = 2; SPH_DISPATCH_K(KERN, CALL); }    \
-            else { constexpr int D = 3; SPH_DISPATCH_K(KERN, CALL); }             \
+            if (DIM == 2) { constexpr int D = 2; SPH_DISPATCH_K(KERN, __VA_ARGS__); }    \
+            else { constexpr int D = 3; SPH_DISPATCH_K(KERN, __VA_ARGS__); }             \
         }                                                                         \
     } while (0)
-#define SPH_DISPATCH_K(KERN, CALL)                                                \
+#define SPH_DISPATCH_K(KERN, ...)                                                \
     switch (KERN) {                                                               \
-        case SPH_KERNEL_GAUSSIAN: { constexpr int K = SPH_KERNEL_GAUSSIAN; CALL; break; } \
-        case SPH_KERNEL_LUCY: { constexpr int K = SPH_KERNEL_LUCY; CALL; break; }         \
-        case SPH_KERNEL_DEBRUN: { constexpr int K = SPH_KERNEL_DEBRUN; CALL; break; }     \
-        default: { constexpr int K = SPH_KERNEL_CUBIC; CALL; break; }                     \
+        case SPH_KERNEL_GAUSSIAN: { constexpr int K = SPH_KERNEL_GAUSSIAN; __VA_ARGS__; break; } \
+        case SPH_KERNEL_LUCY: { constexpr int K = SPH_KERNEL_LUCY; __VA_ARGS__; break; }         \
+        case SPH_KERNEL_DEBRUN: { constexpr int K = SPH_KERNEL_DEBRUN; __VA_ARGS__; break; }     \
+        default: { constexpr int K = SPH_KERNEL_CUBIC; __VA_ARGS__; break; }                     \
     }
 
 }  // namespace sph

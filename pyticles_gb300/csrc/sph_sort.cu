@@ -105,8 +105,9 @@ __global__ void k_scan_reduce(const int *count, int n, int *block_tmp, const int
     if (threadIdx.x == 0) block_tmp[blockIdx.x] = total;
 }
 
-__global__ void k_scan_top(int *block_tmp, int nb, const int *gate) {
+__global__ void k_scan_top(int *block_tmp, int nb, const int *gate, int *clear) {
     if (gate && *gate == 0) return;
+    if (clear && threadIdx.x == 0) *clear = 0;
     // single block, sequential chunks of 1024
     int carry = 0;
     for (int base = 0; base < nb; base += kScanBlock) {
@@ -144,11 +145,11 @@ __global__ void k_scan_apply(const int *count, int *start, int n, const int *blo
 }
 
 void launch_scan(int *count, int *start, int n, int *block_tmp, cudaStream_t s,
-                 const int *gate) {
+                 const int *gate, int *clear) {
     int nb = (n + kScanTile - 1) / kScanTile;
     if (nb < 1) nb = 1;
     k_scan_reduce<<<nb, kScanBlock, 0, s>>>(count, n, block_tmp, gate);
-    k_scan_top<<<1, kScanBlock, 0, s>>>(block_tmp, nb, gate);
+    k_scan_top<<<1, kScanBlock, 0, s>>>(block_tmp, nb, gate, clear);
     k_scan_apply<<<nb, kScanBlock, 0, s>>>(count, start, n, block_tmp, nb, gate);
 }
 
@@ -189,6 +190,19 @@ __global__ void k_cellsort(View v, int ncells) {
             for (int t = 0; t < m; ++t) r += (v.a_id[v.order_tmp[b + t]] < key) ? 1 : 0;
             v.order[b + r] = val;
             v.cell_b[b + r] = cell;
+        }
+        // the cell's work items for the cell tiles
+        if (lane == 0 && m > 0 && v.n_tile > 0) {
+            const SimDev &S = v.sims[v.a_sim[v.order_tmp[b]]];
+            if (S.tile_on) {
+                const int per = kTileRounds * (32 >> S.tile_lg), k = (m + per - 1) / per;
+                const int at = atomicAdd(v.n_items, k);
+                for (int t = 0; t < k; ++t) {
+                    if (!SPH_IN_BOUNDS(at + t < v.np, v.err_any)) break;
+                    v.item_cell[at + t] = cell;
+                    v.item_round[at + t] = t * kTileRounds;
+                }
+            }
         }
     }
 }
