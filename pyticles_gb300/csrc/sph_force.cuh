@@ -204,11 +204,12 @@ __device__ __forceinline__ void integrate_stage(const View &v, const SimDev &S, 
 // single 2D simulation, with its constants out of registers, runs best at 51
 // (5 blocks), 3D at 64.
 // LIST: the pair lists (tuning.pair_scheme 2) instead of the cell windows.
-template <typename R, int D, int K, int VH, bool ONE, bool LIST = false>
+// LANES: lanes per particle (for_pairs_lanes; the same bits).
+template <typename R, int D, int K, int VH, bool ONE, bool LIST = false, int LANES = 1>
 __device__ __forceinline__ void force_one(const View &v, int stage, int mode, int integ, int i) {
     constexpr bool visc = (VH & 1) != 0;
     constexpr bool heat = (VH & 2) != 0;
-    const bool active = i < v.np;
+    bool active = i < v.np;
     const int ii = active ? i : v.np - 1;
     using T4 = typename V4<R>::T;
     const T4 *__restrict__ P = (const T4 *)v.pk_pos_in;
@@ -217,7 +218,10 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
     const T4 *__restrict__ Q = (const T4 *)v.pk_q;
     const int s = v.b_sim[ii];
     const SimDev &S = ONE ? v.one : v.sims[s];
-    if (S.cl_on || (!LIST && S.tile_on)) return;   // cluster passes, cell tiles
+    if (S.cl_on || (!LIST && S.tile_on)) {   // cluster passes, cell tiles
+        if (LANES == 1) return;
+        active = false;
+    }
     KConst<R> ks = make_kconst<R>(S, 0);
     // the long kernel with pco_i/rho_l,i^2 + pco_j/rho_l,j^2 = -2a folded in
     KConst<R> kl = make_kconst_cohesive<R>(S);
@@ -281,11 +285,20 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
         if (D == 3) ax[2].flush();
         ud.flush();
     };
-    if (!active) return;
+    if (LANES == 1 && !active) return;
     {
         PairFrame<R, D> fr;
         fr.init(S);
-        if constexpr (LIST) for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done);
+        if constexpr (LANES > 1) {
+            for_pairs_lanes<R, D, LANES, false>(v, S, fr, P, ii, P[ii], active, body,
+                                                [&](unsigned mask) {
+                                                    fold_lanes<LANES>(ax[0], mask);
+                                                    fold_lanes<LANES>(ax[1], mask);
+                                                    if (D == 3) fold_lanes<LANES>(ax[2], mask);
+                                                    fold_lanes<LANES>(ud, mask);
+                                                });
+            if (!active || (threadIdx.x & (LANES - 1))) return;
+        } else if constexpr (LIST) for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done);
         else for_pairs<R, D, D == 3, false>(v, S, fr, P, i, P[i], body, cell_done);
     }
     R vdr[3] = {ax[0].get(), ax[1].get(), ax[2].get()};
@@ -330,6 +343,14 @@ __global__ void __launch_bounds__(256, ONE ? (D == 2 ? SPH_VL_FORCE_BLOCKS : SPH
                                           blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+// The cell windows of a small launch, LANES lanes per particle.
+template <int D, int K, int VH, int LANES>
+__global__ void __launch_bounds__(256)
+    k_force_lanes(const __grid_constant__ View v, int stage, int mode, int integ) {
+    force_one<float, D, K, VH, false, false, LANES>(
+        v, stage, mode, integ, (blockIdx.x * blockDim.x + threadIdx.x) / LANES);
+}
+
 // Integrator stage from the stored rates: the epilogue of k_force as a pass
 // of its own, for steps whose velocities change between the force pass and
 // the update (hard collisions).
@@ -349,13 +370,18 @@ __global__ void __launch_bounds__(256) k_integrate(View v, int stage, int integ,
 // own (sph_force_*.cu) per dimension.  The persistent form is for the
 // mixed-precision pass only (see density_launch); FP64 walks serve the
 // simulations that are too sparse for cell tiles.
-enum ForceForm { kForceWalk, kForceList };
+enum ForceForm { kForceWalk, kForceList, kForceLanes };
 
 template <int FORM, typename R, int D, int K, int VH, bool ONE>
 void force_launch(const View &v, int stage, int mode, int integ, int block, cudaStream_t s) {
     const int grid = (v.np + block - 1) / block;
     if constexpr (FORM == kForceList) {
         k_force_vl<D, K, VH, ONE><<<grid, block, 0, s>>>(v, stage, mode, integ);
+    } else if constexpr (FORM == kForceLanes) {
+        if (walk_lanes(v) == 32)
+            k_force_lanes<D, K, VH, 32><<<lanes_grid(v, 32), 128, 0, s>>>(v, stage, mode, integ);
+        else
+            k_force_lanes<D, K, VH, 8><<<lanes_grid(v, 8), 128, 0, s>>>(v, stage, mode, integ);
     } else if (std::is_same<R, float>::value && v.persist) {
         auto *fn = k_force<R, D, K, VH, ONE, std::is_same<R, float>::value>;
         fn<<<pass_grid(v, fn, block), block, 0, s>>>(v, stage, mode, integ);
@@ -369,7 +395,7 @@ void launch_force_t(const View &v, int kernel, int viscosity, int heat, int inte
                     int mode, int block, cudaStream_t s) {
     const int vh = (viscosity ? 1 : 0) | (heat ? 2 : 0);
     // constants from the kernel parameters for a single simulation
-    constexpr bool kOne = std::is_same<R, float>::value;
+    constexpr bool kOne = std::is_same<R, float>::value && FORM != kForceLanes;
 #define SPH_FORCE(VH_)                                                                        \
     (v.one_sim && kOne                                                                        \
          ? force_launch<FORM, R, D, K, VH_, kOne>(v, stage, mode, integrator, block, s)       \

@@ -11,6 +11,8 @@ SPH_FORM(kForceWalk, float, 2);
 SPH_FORM(kForceWalk, float, 3);
 SPH_FORM(kForceList, float, 2);
 SPH_FORM(kForceList, float, 3);
+SPH_FORM(kForceLanes, float, 2);
+SPH_FORM(kForceLanes, float, 3);
 SPH_FORM(kForceWalk, double, 2);
 SPH_FORM(kForceWalk, double, 3);
 #undef SPH_FORM
@@ -28,6 +30,8 @@ void launch_force(const View &v, int precision, int kernel, int viscosity, int h
             run(launch_force_t<kForceWalk, double, 2>, launch_force_t<kForceWalk, double, 3>);
     } else if (v.vl_on) {
         run(launch_force_t<kForceList, float, 2>, launch_force_t<kForceList, float, 3>);
+    } else if (walk_lanes(v) > 1) {
+        run(launch_force_t<kForceLanes, float, 2>, launch_force_t<kForceLanes, float, 3>);
     } else {
         run(launch_force_t<kForceWalk, float, 2>, launch_force_t<kForceWalk, float, 3>);
     }

@@ -19,15 +19,19 @@ namespace sph {
 // 32 registers (7 blocks, 60 B spilled), measured 6.3% faster than 48 and 2%
 // faster than 40; 3D and FP64 at 51.
 // LIST: the pair lists (tuning.pair_scheme 2) instead of the cell windows.
-template <typename R, int D, int K, bool ONE, bool LIST = false>
+// LANES: lanes per particle (for_pairs_lanes; the same bits).
+template <typename R, int D, int K, bool ONE, bool LIST = false, int LANES = 1>
 __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
-    const bool active = i < v.np;
+    bool active = i < v.np;
     const int ii = active ? i : v.np - 1;
     using T4 = typename V4<R>::T;
     const T4 *__restrict__ P = (const T4 *)v.pk_pos_in;
     const int s = v.b_sim[ii];
     const SimDev &S = ONE ? v.one : v.sims[s];
-    if (S.cl_on || (!LIST && S.tile_on)) return;   // cluster passes, cell tiles
+    if (S.cl_on || (!LIST && S.tile_on)) {   // cluster passes, cell tiles
+        if (LANES == 1) return;
+        active = false;
+    }
     KConst<R> ks = make_kconst<R>(S, 0);
     KConst<R> kl = make_kconst<R>(S, 1);
     BAcc<R> rs, rl;
@@ -49,11 +53,20 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
         rs.flush();
         rl.flush();
     };
-    if (!active) return;
+    if (LANES == 1 && !active) return;
     {
         PairFrame<R, D> fr;
         fr.init(S);
-        if constexpr (LIST) {
+        if constexpr (LANES > 1) {
+            for_pairs_lanes<R, D, LANES, true>(v, S, fr, P, ii, P[ii], active, body,
+                                               [&](unsigned mask) {
+                                                   fold_lanes<LANES>(rs, mask);
+                                                   fold_lanes<LANES>(rl, mask);
+                                               });
+#pragma unroll
+            for (int o = LANES / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+            if (!active || (threadIdx.x & (LANES - 1))) return;
+        } else if constexpr (LIST) {
             for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done);
         } else {
             for_pairs<R, D>(v, S, fr, P, i, P[i], body, cell_done);
@@ -94,16 +107,19 @@ __global__ void __launch_bounds__(256, ONE ? (D == 2 ? SPH_VL_DENSITY_BLOCKS : S
 }
 
 // At most 64 registers (4 blocks of 256 per SM): 8% faster in 3D than 80.
-template <typename R, int D, int K, bool ONE, bool LIST = false>
+template <typename R, int D, int K, bool ONE, bool LIST = false, int LANES = 1>
 __device__ __forceinline__ void heat_one(const View &v, int i) {
-    const bool active = i < v.np;
+    bool active = i < v.np;
     const int ii = active ? i : v.np - 1;
     using T4 = typename V4<R>::T;
     const T4 *__restrict__ P = (const T4 *)v.pk_pos_in;
     const T4 *__restrict__ F = (const T4 *)v.pk_f;
     const int s = v.b_sim[ii];
     const SimDev &S = ONE ? v.one : v.sims[s];
-    if (S.cl_on || (!LIST && S.tile_on)) return;   // cluster passes, cell tiles
+    if (S.cl_on || (!LIST && S.tile_on)) {   // cluster passes, cell tiles
+        if (LANES == 1) return;
+        active = false;
+    }
     KConst<R> ks = make_kconst<R>(S, 0);
     const T4 fi = F[ii];
     BAcc<R> q[3];
@@ -124,14 +140,22 @@ __device__ __forceinline__ void heat_one(const View &v, int i) {
         q[1].flush();
         if (D == 3) q[2].flush();
     };
-    if (!active) return;
+    if (LANES == 1 && !active) return;
     {
         PairFrame<R, D> fr;
         fr.init(S);
         // only the short kernel enters q: cells and pairs beyond its support
         // contribute exactly zero and are not visited
         fr.thr_hi = fr.thr_s;
-        if constexpr (LIST) for_list<R, D, false>(v, S, fr, P, i, P[i], body, cell_done);
+        if constexpr (LANES > 1) {
+            for_pairs_lanes<R, D, LANES, false>(v, S, fr, P, ii, P[ii], active, body,
+                                                [&](unsigned mask) {
+                                                    fold_lanes<LANES>(q[0], mask);
+                                                    fold_lanes<LANES>(q[1], mask);
+                                                    if (D == 3) fold_lanes<LANES>(q[2], mask);
+                                                });
+            if (!active || (threadIdx.x & (LANES - 1))) return;
+        } else if constexpr (LIST) for_list<R, D, false>(v, S, fr, P, i, P[i], body, cell_done);
         else for_pairs<R, D, D == 3, false>(v, S, fr, P, i, P[i], body, cell_done);
     }
     R kap = sconst<R>(S).kappa;
@@ -158,6 +182,21 @@ __global__ void __launch_bounds__(256, 4) k_heat_vl(const __grid_constant__ View
     heat_one<float, D, K, ONE, true>(v, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+// The cell windows of a small mixed-precision launch, LANES lanes per particle:
+// one thread per particle would leave most SMs without a warp (1,024
+// particles: eight warps of 32) and every lane with the window's whole chain.
+// The epilogue runs on the first lane of each particle.
+template <int D, int K, int LANES>
+__global__ void __launch_bounds__(256) k_density_lanes(const __grid_constant__ View v, int stage) {
+    density_one<float, D, K, false, false, LANES>(
+        v, stage, (blockIdx.x * blockDim.x + threadIdx.x) / LANES);
+}
+template <int D, int K, int LANES>
+__global__ void __launch_bounds__(256) k_heat_lanes(const __grid_constant__ View v) {
+    heat_one<float, D, K, false, false, LANES>(v,
+                                               (blockIdx.x * blockDim.x + threadIdx.x) / LANES);
+}
+
 // The persistent form is instantiated for the mixed-precision passes only;
 // FP64 engines launch one thread per particle whatever tuning.persistent says.
 // Pair lists (v.vl_on) exist for mixed-precision engines only.
@@ -166,6 +205,15 @@ void density_launch(const View &v, int stage, int block, cudaStream_t s) {
     if constexpr (std::is_same<R, float>::value) {
         if (v.vl_on) {
             k_density_vl<D, K, ONE><<<(v.np + block - 1) / block, block, 0, s>>>(v, stage);
+            return;
+        }
+        const int lanes = walk_lanes(v);
+        if (lanes == 32) {
+            k_density_lanes<D, K, 32><<<lanes_grid(v, 32), 128, 0, s>>>(v, stage);
+            return;
+        }
+        if (lanes == 8) {
+            k_density_lanes<D, K, 8><<<lanes_grid(v, 8), 128, 0, s>>>(v, stage);
             return;
         }
     }
@@ -182,6 +230,15 @@ void heat_launch(const View &v, int block, cudaStream_t s) {
     if constexpr (std::is_same<R, float>::value) {
         if (v.vl_on) {
             k_heat_vl<D, K, ONE><<<(v.np + block - 1) / block, block, 0, s>>>(v);
+            return;
+        }
+        const int lanes = walk_lanes(v);
+        if (lanes == 32) {
+            k_heat_lanes<D, K, 32><<<lanes_grid(v, 32), 128, 0, s>>>(v);
+            return;
+        }
+        if (lanes == 8) {
+            k_heat_lanes<D, K, 8><<<lanes_grid(v, 8), 128, 0, s>>>(v);
             return;
         }
     }

@@ -71,6 +71,74 @@ template <typename R> __device__ __forceinline__ R fmaxf_(R c, R ext) {
     return a > (R)0 ? a : (R)0;
 }
 
+// One window cell of particle i (linear cell lin, offset (ox, oy, oz)): body for
+// every pair of i in it, in cell order.  near_cell: the cell may hold pairs
+// within the short support.  Returns whether the cell was scanned.
+template <typename R, int D, bool PF, bool SELF, typename T4, typename F>
+__device__ __forceinline__ bool pair_cell(const View &v, const SimDev &S,
+                                          const PairFrame<R, D> &fr, const T4 *__restrict__ P,
+                                          int i, const T4 &pi, const int *mort, int lin, int ox,
+                                          int oy, int oz, bool near_cell, F &body) {
+    if (!SPH_IN_BOUNDS(lin >= 0 && lin < S.ncells, v.err_any)) return false;
+    const int gc = S.cell_off + mort[lin];
+    if (!SPH_IN_BOUNDS(gc >= S.cell_off && gc < S.cell_off + S.ncells, v.err_any)) return false;
+    // offset of the window cell's frame from particle i; in FP32
+    // the cell edge is a hi/lo pair, so that the offset carries one
+    // rounding instead of the edge's rounding times the cell count
+    R ox_ = (R)ox * fr.edge[0] - pi.x;
+    R oy_ = (R)oy * fr.edge[1] - pi.y;
+    R oz_ = (D == 3) ? (R)oz * fr.edge[2] - pi.z : (R)0;
+    if constexpr (std::is_same<R, float>::value) {
+        ox_ = __fmaf_rn((R)ox, fr.edge_lo[0], ox_);
+        oy_ = __fmaf_rn((R)oy, fr.edge_lo[1], oy_);
+        if (D == 3) oz_ = __fmaf_rn((R)oz, fr.edge_lo[2], oz_);
+    }
+    const int jb = v.cell_start[gc], je = v.cell_start[gc + 1];
+    if (!SPH_IN_BOUNDS(jb >= 0 && jb <= je && je <= v.np, v.err_any)) return false;
+    auto scan = [&](auto near, auto self, auto mi) {
+        T4 pn;
+        if (PF) pn = P[jb < je ? jb : i];
+        for (int j = jb; j < je; ++j) {
+            T4 pj;
+            if (PF) {
+                pj = pn;
+                if (j + 1 < je) pn = P[j + 1];
+            }
+            if (decltype(self)::value && j == i) continue;
+            if (!PF) pj = P[j];
+            R d[3];
+            d[0] = pj.x + ox_;
+            d[1] = pj.y + oy_;
+            d[2] = (D == 3) ? pj.z + oz_ : (R)0;
+            if constexpr (decltype(mi)::value) fr.min_image(d);
+            R rsq = d[0] * d[0] + d[1] * d[1];
+            if (D == 3) rsq += d[2] * d[2];
+            if (rsq > fr.thr_hi) continue;
+            if (rsq >= fr.thr_lo && !exact_in_set<D>(v.xe_in, &S, i, j)) continue;
+            body(j, pj, d, rsq, near);
+        }
+    };
+    // the minimum image applies only on single-cell axes: the scan
+    // is compiled with and without it (4.7% of the 2D density
+    // pass, which otherwise tested small_mask per candidate)
+    if (fr.small_mask) {
+        if (SELF && ox == 0 && oy == 0 && oz == 0)
+            scan(std::true_type{}, std::true_type{}, std::true_type{});
+        else if (__any_sync(__activemask(), near_cell))
+            scan(std::true_type{}, std::false_type{}, std::true_type{});
+        else
+            scan(std::false_type{}, std::false_type{}, std::true_type{});
+    } else {
+        if (SELF && ox == 0 && oy == 0 && oz == 0)
+            scan(std::true_type{}, std::true_type{}, std::false_type{});
+        else if (__any_sync(__activemask(), near_cell))
+            scan(std::true_type{}, std::false_type{}, std::false_type{});
+        else
+            scan(std::false_type{}, std::false_type{}, std::false_type{});
+    }
+    return true;
+}
+
 // Iterates the pair set of particle i.  body(j, pj, d[3], rsq, near) is called
 // for every j != i that passes the exact pair test, in a fixed order: neighbour
 // cells in raster order (z, y, x) of their offset from i's cell, particles in
@@ -129,68 +197,74 @@ __device__ __forceinline__ void for_pairs(const View &v, const SimDev &S,
                 int x = c0 + ox;
                 x += (x < 0) ? n0 : 0;
                 x -= (x >= n0) ? n0 : 0;
-                if (!SPH_IN_BOUNDS(row + x >= 0 && row + x < S.ncells, v.err_any)) continue;
-                const int gc = S.cell_off + mort[row + x];
-                if (!SPH_IN_BOUNDS(gc >= S.cell_off && gc < S.cell_off + S.ncells, v.err_any))
-                    continue;
-                // offset of the window cell's frame from particle i; in FP32
-                // the cell edge is a hi/lo pair, so that the offset carries one
-                // rounding instead of the edge's rounding times the cell count
-                R ox_ = (R)ox * fr.edge[0] - pi.x;
-                R oy_ = (R)oy * fr.edge[1] - pi.y;
-                R oz_ = (D == 3) ? (R)oz * fr.edge[2] - pi.z : (R)0;
-                if constexpr (std::is_same<R, float>::value) {
-                    ox_ = __fmaf_rn((R)ox, fr.edge_lo[0], ox_);
-                    oy_ = __fmaf_rn((R)oy, fr.edge_lo[1], oy_);
-                    if (D == 3) oz_ = __fmaf_rn((R)oz, fr.edge_lo[2], oz_);
-                }
-                const int jb = v.cell_start[gc], je = v.cell_start[gc + 1];
-                if (!SPH_IN_BOUNDS(jb >= 0 && jb <= je && je <= v.np, v.err_any)) continue;
-                auto scan = [&](auto near, auto self, auto mi) {
-                    T4 pn;
-                    if (PF) pn = P[jb < je ? jb : i];
-                    for (int j = jb; j < je; ++j) {
-                        T4 pj;
-                        if (PF) {
-                            pj = pn;
-                            if (j + 1 < je) pn = P[j + 1];
-                        }
-                        if (decltype(self)::value && j == i) continue;
-                        if (!PF) pj = P[j];
-                        R d[3];
-                        d[0] = pj.x + ox_;
-                        d[1] = pj.y + oy_;
-                        d[2] = (D == 3) ? pj.z + oz_ : (R)0;
-                        if constexpr (decltype(mi)::value) fr.min_image(d);
-                        R rsq = d[0] * d[0] + d[1] * d[1];
-                        if (D == 3) rsq += d[2] * d[2];
-                        if (rsq > fr.thr_hi) continue;
-                        if (rsq >= fr.thr_lo && !exact_in_set<D>(v.xe_in, &S, i, j)) continue;
-                        body(j, pj, d, rsq, near);
-                    }
-                };
-                // the minimum image applies only on single-cell axes: the scan
-                // is compiled with and without it (4.7% of the 2D density
-                // pass, which otherwise tested small_mask per candidate)
-                if (fr.small_mask) {
-                    if (SELF && ox == 0 && oy == 0 && oz == 0)
-                        scan(std::true_type{}, std::true_type{}, std::true_type{});
-                    else if (__any_sync(__activemask(), dx * dx + dyz < fr.thr_s))
-                        scan(std::true_type{}, std::false_type{}, std::true_type{});
-                    else
-                        scan(std::false_type{}, std::false_type{}, std::true_type{});
-                } else {
-                    if (SELF && ox == 0 && oy == 0 && oz == 0)
-                        scan(std::true_type{}, std::true_type{}, std::false_type{});
-                    else if (__any_sync(__activemask(), dx * dx + dyz < fr.thr_s))
-                        scan(std::true_type{}, std::false_type{}, std::false_type{});
-                    else
-                        scan(std::false_type{}, std::false_type{}, std::false_type{});
-                }
-                cell_done();
+                if (pair_cell<R, D, PF, SELF>(v, S, fr, P, i, pi, mort, row + x, ox, oy, oz,
+                                              dx * dx + dyz < fr.thr_s, body))
+                    cell_done();
             }
         }
     }
+}
+
+// for_pairs with G lanes per particle (G = 8 or 32 consecutive lanes, all of
+// the warp's lanes calling): lane l scans the window cells l, l + G, ... and
+// fold(mask) then adds the G cells' blocked sums in raster order, mask holding
+// the lanes whose cell was scanned.  The terms of a cell are summed by one
+// lane and the cells folded in for_pairs' order, so the sums carry for_pairs'
+// bits: the launch's size may choose between the two.
+template <typename R, int D, int G, bool SELF, typename T4, typename F, typename H>
+__device__ __forceinline__ void for_pairs_lanes(const View &v, const SimDev &S,
+                                                const PairFrame<R, D> &fr,
+                                                const T4 *__restrict__ P, int i, const T4 &pi,
+                                                bool active, F body, H fold) {
+    const int lane = threadIdx.x & 31, l = lane & (G - 1);
+    const int cp = v.cell_xyz[v.cell_b[i]];
+    const int c0 = cp & 2047, c1 = (cp >> 11) & 2047, c2 = (cp >> 22) & 1023;
+    const int w0 = S.win[0], w1 = S.win[1], w2 = D == 3 ? S.win[2] : 0;
+    const int e0 = 2 * w0 + 1, e1 = 2 * w1 + 1;
+    const int n0 = S.nc[0], n1 = S.nc[1], n2 = S.nc[2];
+    const int *mort = v.morton + S.cell_off;
+    const int ncw = active ? e0 * e1 * (2 * w2 + 1) : 0;
+    // the particles of a warp may belong to simulations with other windows
+    const int rounds = __reduce_max_sync(0xffffffffu, (ncw + G - 1) / G);
+    for (int r = 0; r < rounds; ++r) {
+        const int c = r * G + l;
+        bool scanned = false;
+        if (c < ncw) {
+            const int row = c / e0, ox = c - row * e0 - w0;
+            const int oy = (D == 3 ? row % e1 : row) - w1, oz = D == 3 ? row / e1 - w2 : 0;
+            const R dx = fmaxf_((R)ox * fr.edge[0] - pi.x, fr.ext[0]);
+            const R dy = fmaxf_((R)oy * fr.edge[1] - pi.y, fr.ext[1]);
+            const R dz = D == 3 ? fmaxf_((R)oz * fr.edge[2] - pi.z, fr.ext[2]) : (R)0;
+            const R dyz = dy * dy + dz * dz;
+            if (!(dyz > fr.thr_hi) && !(dx * dx + dyz > fr.thr_hi)) {
+                int x = c0 + ox, y = c1 + oy, z = D == 3 ? c2 + oz : 0;
+                x += x < 0 ? n0 : 0;
+                x -= x >= n0 ? n0 : 0;
+                y += y < 0 ? n1 : 0;
+                y -= y >= n1 ? n1 : 0;
+                if (D == 3) {
+                    z += z < 0 ? n2 : 0;
+                    z -= z >= n2 ? n2 : 0;
+                }
+                scanned = pair_cell<R, D, false, SELF>(v, S, fr, P, i, pi, mort,
+                                                       (z * n1 + y) * n0 + x, ox, oy, oz,
+                                                       dx * dx + dyz < fr.thr_s, body);
+            }
+        }
+        fold((__ballot_sync(0xffffffffu, scanned) >> (lane & ~(G - 1))) &
+             (G == 32 ? 0xffffffffu : (1u << G) - 1u));
+    }
+}
+
+// Adds the G lanes' blocks of a sum in lane order, on every lane: the lanes in
+// mask as BAcc::flush would.
+template <int G> __device__ __forceinline__ void fold_lanes(BAcc<float> &a, unsigned mask) {
+#pragma unroll 8
+    for (int c = 0; c < G; ++c) {
+        const float x = __shfl_sync(0xffffffffu, a.part, c, G);
+        if (mask & (1u << c)) a.total.add(x);
+    }
+    a.part = 0.0f;
 }
 
 // Window offset k - 3 of a list entry's 3-bit field k, as an exact float:
@@ -289,6 +363,17 @@ template <typename F> inline int pass_grid(const View &v, F *kernel, int block) 
     if (!v.persist) return nb;
     const int cap = resident_blocks((const void *)kernel, block);
     return nb < cap ? nb : cap;
+}
+
+// Lanes per particle of the mixed-precision cell-window passes, by the
+// particles of the launch (the bits do not depend on it).  All pair passes of a
+// step, us, with 1 / 8 / 32 lanes: 2D 1,024 particles 340 / 111 / 73, 4,096 325 /
+// 108 / 107, 16,384 352 / 185 / 247, 32,761 350 / 259 / 432, 65,536 375 / 432 /
+// 816; 3D with heat flux 2,197 particles 2122 / 615 / 274, 8,000 2124 / 608 / 675,
+// 32,768 2354 / 1923 / 2505, 64,000 2377 / 3041 / 4484.
+inline int walk_lanes(const View &v) { return v.np <= 4096 ? 32 : (v.np <= 40960 ? 8 : 1); }
+inline int lanes_grid(const View &v, int lanes) {   // blocks of 128 threads
+    return (int)(((long long)v.np * lanes + 127) / 128);
 }
 
 // Warp-aggregated per-simulation counter update.
