@@ -298,7 +298,7 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
                                                     fold_lanes<LANES>(ud, mask);
                                                 });
             if (!active || (threadIdx.x & (LANES - 1))) return;
-        } else if constexpr (LIST) for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done);
+        } else if constexpr (LIST) for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done, [] {});
         else for_pairs<R, D, D == 3, false>(v, S, fr, P, i, P[i], body, cell_done);
     }
     R vdr[3] = {ax[0].get(), ax[1].get(), ax[2].get()};

@@ -47,7 +47,7 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
         }
         kernel_wg<K, R>(kl, dd, &w, &g);
         rl.add(pj.w * w);
-        ++cnt;
+        if (!LIST) ++cnt;
     };
     auto cell_done = [&]() {
         rs.flush();
@@ -67,7 +67,10 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
             for (int o = LANES / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
             if (!active || (threadIdx.x & (LANES - 1))) return;
         } else if constexpr (LIST) {
-            for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done);
+            // the entries of whole groups, less those that are no pairs
+            const unsigned c = v.vl_cnt[i];
+            cnt = (((c & 0xffffu) + 3) & ~3u) + (((c >> 16) + 3) & ~3u);
+            for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done, [&]() { --cnt; });
         } else {
             for_pairs<R, D>(v, S, fr, P, i, P[i], body, cell_done);
         }
@@ -147,6 +150,7 @@ __device__ __forceinline__ void heat_one(const View &v, int i) {
         // only the short kernel enters q: cells and pairs beyond its support
         // contribute exactly zero and are not visited
         fr.thr_hi = fr.thr_s;
+        fr.thr_lo = fr.thr_lo < fr.thr_s ? fr.thr_lo : fr.thr_s;
         if constexpr (LANES > 1) {
             for_pairs_lanes<R, D, LANES, false>(v, S, fr, P, ii, P[ii], active, body,
                                                 [&](unsigned mask) {
@@ -155,7 +159,7 @@ __device__ __forceinline__ void heat_one(const View &v, int i) {
                                                     if (D == 3) fold_lanes<LANES>(q[2], mask);
                                                 });
             if (!active || (threadIdx.x & (LANES - 1))) return;
-        } else if constexpr (LIST) for_list<R, D, false>(v, S, fr, P, i, P[i], body, cell_done);
+        } else if constexpr (LIST) for_list<R, D, false>(v, S, fr, P, i, P[i], body, cell_done, [] {});
         else for_pairs<R, D, D == 3, false>(v, S, fr, P, i, P[i], body, cell_done);
     }
     R kap = sconst<R>(S).kappa;

@@ -290,10 +290,15 @@ __device__ __forceinline__ float vl_offset(unsigned k) {
 // The separation is rebuilt from the entry's window offset: d = (p_j - p_i)
 // + o e + o e_lo with the cell edge as a hi/lo pair, every rounding at the
 // magnitude of d.
-template <typename R, int D, bool FAR, typename T4, typename F, typename G>
+//
+// Every run fills whole groups: the build ends it with entries that name the
+// particle itself three window cells away on every axis, which no pair within
+// the cutoff is, so that the walk tests no entry's place.  skip() is called for
+// every entry that is no pair, these among them.
+template <typename R, int D, bool FAR, typename T4, typename F, typename G, typename H>
 __device__ __forceinline__ void for_list(const View &v, const SimDev &S,
                                          const PairFrame<R, D> &fr, const T4 *__restrict__ P,
-                                         int i, const T4 &pi, F body, G cell_done) {
+                                         int i, const T4 &pi, F body, G cell_done, H skip) {
     static_assert(std::is_same<R, float>::value, "pair lists: mixed precision");
     constexpr int kBits = vl_index_bits(D);
     const unsigned cnt = v.vl_cnt[i];
@@ -316,30 +321,32 @@ __device__ __forceinline__ void for_list(const View &v, const SimDev &S,
             d[2] = __fmaf_rn(fz, fr.edge_lo[2], __fmaf_rn(fz, fr.edge[2], __fsub_rn(pj.z, pi.z)));
             rsq += d[2] * d[2];
         }
-        if (rsq > fr.thr_hi) return;
-        if (rsq >= fr.thr_lo && !exact_in_set<D>(v.xe_in, &S, i, j)) return;
+        // one branch for the guard band and everything beyond it
+        if (rsq >= fr.thr_lo && (rsq > fr.thr_hi || !exact_in_set<D>(v.xe_in, &S, i, j))) {
+            skip();
+            return;
+        }
         body(j, pj, d, rsq, near);
     };
-    // n entries from group pointer g, stepping `dir` rows per group; slots
-    // in order 0..3 (near) or 3..0 (far).  Measured on the 2D fluid: a
-    // lookahead of one group is enough (two, or the group's four records
-    // loaded ahead of their tests, were 3-6% slower: more registers)
+    // the groups from pointer g, stepping `dir` rows each; slots in order
+    // 0..3 (near) or 3..0 (far).  Measured on the 2D fluid: a lookahead of
+    // one group is enough (two, or the group's four records loaded ahead of
+    // their tests, were 3-6% slower: more registers)
     auto walk = [&](const int4 *g, long long dir, int n, auto near, auto rev) {
         const int ng = (n + 3) >> 2;
         int4 cur = ng > 0 ? *g : make_int4(0, 0, 0, 0);
         for (int k = 0; k < ng; ++k) {
             const int4 nxt = k + 1 < ng ? g[(k + 1) * dir] : cur;
-            const int left = n - 4 * k;
             if constexpr (decltype(rev)::value) {
                 one(cur.w, near);
-                if (left > 1) one(cur.z, near);
-                if (left > 2) one(cur.y, near);
-                if (left > 3) one(cur.x, near);
+                one(cur.z, near);
+                one(cur.y, near);
+                one(cur.x, near);
             } else {
                 one(cur.x, near);
-                if (left > 1) one(cur.y, near);
-                if (left > 2) one(cur.z, near);
-                if (left > 3) one(cur.w, near);
+                one(cur.y, near);
+                one(cur.z, near);
+                one(cur.w, near);
             }
             if ((k & 3) == 3) cell_done();
             cur = nxt;

@@ -123,14 +123,17 @@ __global__ void __launch_bounds__(256) k_vlist_build(const __grid_constant__ Vie
             }
         }
         if (store) {
-            // the partial last groups, shifted into place (their unused
-            // slots are never read)
+            // the partial last groups, filled up with the particle itself
+            // three window cells away on every axis: further than the
+            // cutoff, whatever the window (a cell spans at least a third of
+            // the cutoff plus the skin)
+            const int none = i | (int)((D == 3 ? 0x1b6u : 0x36u) << kBits);
             if (wn & 3) {
-                for (int t = wn & 3; t < 4; ++t) gn = make_int4(gn.y, gn.z, gn.w, 0);
+                for (int t = wn & 3; t < 4; ++t) gn = make_int4(gn.y, gn.z, gn.w, none);
                 rows[(long long)(wn >> 2) * l.stride] = gn;
             }
             if (wf & 3) {
-                for (int t = wf & 3; t < 4; ++t) gf = make_int4(0, gf.x, gf.y, gf.z);
+                for (int t = wf & 3; t < 4; ++t) gf = make_int4(none, gf.x, gf.y, gf.z);
                 rows[far0 - (long long)(wf >> 2) * l.stride] = gf;
             }
             // an overflowing list keeps the entries that fit (the first cap
