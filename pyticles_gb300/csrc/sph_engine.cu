@@ -337,6 +337,25 @@ void fill_const(SimConst<R> &c, const sph_engine *e, const Sim &S, const SimDev 
     c.kappa = (R)p.thermalk;
 }
 
+// Relative half width of the guard band around the cutoff in FP32: four times a
+// bound on what rounding can move an FP32 squared distance at the cutoff.  A
+// position's local coordinate has at most h (half its cell and the allowed
+// drift), a window cell's frame lies at most win edge + h away, and a separation
+// takes at most four roundings of such magnitudes per axis; 16 more units cover
+// the squares and sums.  5e-6 for the 2D fluid (measured error below 1e-6).
+// Every pair inside the band pays the FP64 test with a warp to itself: a band of
+// 2^-12 kept the FP64 pipe of the 3D list density pass 43% busy.
+double fast_margin(const sph_engine *e, const Sim &S, const SimDev &d) {
+    double most = 0.0;
+    for (int a = 0; a < e->dim; ++a) {
+        const double h = S.win[a] > 0 ? d.box_half[a] : 0.5 * d.L[a];
+        const double reach = S.win[a] > 0 ? S.win[a] * S.edge[a] : d.L[a];
+        most = std::max(most, 4.0 * (reach + 3.0 * h));
+    }
+    const double ulp = 1.0 / 16777216.0;
+    return ulp * (16.0 + 4.0 * 2.0 * std::sqrt((double)e->dim) * most / std::sqrt(d.thr));
+}
+
 // Cell tiles serve simulations whose cells hold at least two particles on
 // average (a block fills its tile once per cell, and a nearly empty cell does
 // not repay it).  The rules are of the simulation alone, so its bits are too.
@@ -417,9 +436,7 @@ SimDev make_simdev(const sph_engine *e, const Sim &S) {
                                                   S.edge[a]));
         d.coll_win[a] = w;
     }
-    // fast-test guard band: 2^-12 relative in FP32 (cell-local coordinates
-    // keep the FP32 squared distance within 5e-6 of the FP64 one), 1e-9 in FP64
-    fill_const<float>(d.cf, e, S, d, 1.0 / 4096.0);
+    fill_const<float>(d.cf, e, S, d, fast_margin(e, S, d));
     fill_const<double>(d.cd, e, S, d, 1e-9);
     return d;
 }

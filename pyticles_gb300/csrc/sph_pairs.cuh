@@ -6,7 +6,7 @@
 // cells around its own cell, so each unordered pair is evaluated from both
 // sides and no atomics touch particle data.  Positions are cell-local
 // (relative to the particle's cell centre), which keeps FP32 differences
-// accurate; the pair-set test runs on those FP32 distances with a 2^-12
+// accurate; the pair-set test runs on those FP32 distances with a
 // guard band and falls back to the reference's FP64 test for pairs inside
 // the band, so the pair set is bit-exact.
 #pragma once

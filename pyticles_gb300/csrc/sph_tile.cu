@@ -93,7 +93,7 @@ __device__ __forceinline__ double tile_pos(double x) {
 }
 
 // Whether rsq lies past the guard band's lower end, by the high words: the band
-// is 2^-12 wide, and comparing costs the FP64 pipe as much as adding.
+// is a few 1e-6 wide, and comparing costs the FP64 pipe as much as adding.
 __device__ __forceinline__ bool tile_band(double rsq, double thr_lo) {
     return __double2hiint(rsq) >= __double2hiint(thr_lo);
 }
