@@ -199,10 +199,9 @@ __device__ __forceinline__ void integrate_stage(const View &v, const SimDev &S, 
 // VH: bit 0 viscosity, bit 1 heat flux (compile-time, so a workload without
 // them carries neither their registers nor their branches).  ONE: a single
 // simulation, whose constants come from the kernel parameters.
-// Register caps: 64 (4 blocks of 256 per SM) measured 17% faster than the
-// unconstrained 80-104 despite a few spilled words outside the pair loop; a
-// single 2D simulation, with its constants out of registers, runs best at 51
-// (5 blocks), 3D at 64.
+// Register caps by resident blocks of 256 threads; force of a step, us: a single
+// simulation in 2D (199k particles) 324 / 337 / 294 at 4 / 5 / 6 blocks, in 3D (205k)
+// 2178 / 2248 / 2649 at 3 / 4 / 5; several 623 / 584 / 600 at 3 / 4 / 5.
 // LIST: the pair lists (tuning.pair_scheme 2) instead of the cell windows.
 // LANES: lanes per particle (for_pairs_lanes; the same bits).
 template <typename R, int D, int K, int VH, bool ONE, bool LIST = false, int LANES = 1>
@@ -314,7 +313,7 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
 // One thread per particle; PERSIST: the resident blocks of pass_grid walk
 // the particles grid-stride (the same per-particle work, the same bits).
 template <typename R, int D, int K, int VH, bool ONE, bool PERSIST>
-__global__ void __launch_bounds__(256, (ONE && D == 2) ? 5 : 4) k_force(const __grid_constant__ View v, int stage,
+__global__ void __launch_bounds__(256, ONE ? (D == 2 ? 6 : 3) : 4) k_force(const __grid_constant__ View v, int stage,
                                                   int mode, int integ) {
     if constexpr (PERSIST) {
         for (int base = blockIdx.x * blockDim.x; base < v.np; base += gridDim.x * blockDim.x)

@@ -13,11 +13,10 @@
 
 namespace sph {
 
-// At most 64 registers (4 blocks of 256 per SM): the two loop bodies of
-// for_pairs would otherwise take 80 and cost 5-20% in occupancy.  A single
-// simulation (its constants are kernel parameters): 2D mixed precision at
-// 32 registers (7 blocks, 60 B spilled), measured 6.3% faster than 48 and 2%
-// faster than 40; 3D and FP64 at 51.
+// Register caps by resident blocks of 256 threads.  A single simulation (its
+// constants are kernel parameters) runs best at 6 (40 registers): density of
+// a step, us, at 5 / 6 / 7 blocks 252 / 229 / 233 in 2D (199k particles) and 1625 /
+// 1429 / 1446 in 3D (205k); several at 4 (391 us against 418 at 5).
 // LIST: the pair lists (tuning.pair_scheme 2) instead of the cell windows.
 // LANES: lanes per particle (for_pairs_lanes; the same bits).
 template <typename R, int D, int K, bool ONE, bool LIST = false, int LANES = 1>
@@ -81,7 +80,7 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
 // One thread per particle; PERSIST: the resident blocks of pass_grid walk
 // the particles grid-stride (the same per-particle work, the same bits).
 template <typename R, int D, int K, bool ONE, bool PERSIST>
-__global__ void __launch_bounds__(256, ONE ? ((D == 2 && sizeof(R) == 4) ? 7 : 5) : 4) k_density(const __grid_constant__ View v, int stage) {
+__global__ void __launch_bounds__(256, ONE ? 6 : 4) k_density(const __grid_constant__ View v, int stage) {
     if constexpr (PERSIST) {
         for (int base = blockIdx.x * blockDim.x; base < v.np; base += gridDim.x * blockDim.x)
             density_one<R, D, K, ONE>(v, stage, base + threadIdx.x);
@@ -92,10 +91,12 @@ __global__ void __launch_bounds__(256, ONE ? ((D == 2 && sizeof(R) == 4) ? 7 : 5
 
 // The density pass over the pair lists (mixed precision); a single
 // simulation at SPH_VL_DENSITY_BLOCKS (2D) / SPH_VL_DENSITY3_BLOCKS (3D)
-// resident blocks of 256 per SM, several at SPH_VL_DENSITY_MULTI_BLOCKS
-// (5: 6.5% faster than 4 for 512 batched 2D simulations).
+// resident blocks of 256 per SM, several at SPH_VL_DENSITY_MULTI_BLOCKS.
+// Density of a step, us: 2D 1M particles 531 / 509 / 571 at 5 / 6 / 7 blocks;
+// 3D 2M 4058 / 3997 / 4234 at 5 / 6 / 7; 24 batched simulations 263 / 256 / 260
+// at 4 / 5 / 6.
 #ifndef SPH_VL_DENSITY_BLOCKS
-#define SPH_VL_DENSITY_BLOCKS 7
+#define SPH_VL_DENSITY_BLOCKS 6
 #endif
 #ifndef SPH_VL_DENSITY3_BLOCKS
 #define SPH_VL_DENSITY3_BLOCKS 6
@@ -181,8 +182,9 @@ __global__ void __launch_bounds__(256, 4) k_heat(const __grid_constant__ View v)
     }
 }
 
+// (3D 2M particles, a step: 1230 us at 4 blocks, 1161 at 5, 1269 at 6)
 template <int D, int K, bool ONE>
-__global__ void __launch_bounds__(256, 4) k_heat_vl(const __grid_constant__ View v) {
+__global__ void __launch_bounds__(256, 5) k_heat_vl(const __grid_constant__ View v) {
     heat_one<float, D, K, ONE, true>(v, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
