@@ -12,22 +12,12 @@
 // (spkernel.lucy_w, spkernel.py:54-63) or, for the 3D map of particles onto
 // the plane z, the 3D Lucy kernel.  FP64 throughout; contributions are added
 // with atomics, so the last bits of a pixel may depend on arrival order.
+#include <algorithm>
 #include <cmath>
 
-#include "sph_internal.h"
+#include "sph_device.cuh"
 
 namespace {
-
-__device__ __forceinline__ double lucy_w(double s, double h, int dim3) {
-    const double pi = 3.14159265358979323846;
-    double q = dim3 ? 105.0 / (pi * 16.0 * (h * h * h)) : 5.0 / (pi * h * h);
-    if (s < 0) s = -s;
-    if (s < h) {
-        double t = 1.0 - s / h;
-        return q * (1.0 + 3.0 * s / h) * (t * t * t);
-    }
-    return 0.0;
-}
 
 __device__ __forceinline__ double min_image(double d, double L) {
     if (d > L / 2.) d = d - L;
@@ -35,48 +25,173 @@ __device__ __forceinline__ double min_image(double d, double L) {
     return d;
 }
 
-// one thread per particle; r is n x cols row-major
-__global__ void k_splat(int n, const double *r, int cols, const double *m, const double *rho,
-                        const double *a, const double *h, int nx, int ny, const double *x,
-                        const double *y, double z, double xmin, double xmax, double ymin,
-                        double ymax, double cutoff, int dim3, double *Z) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double rx = r[(size_t)i * cols], ry = r[(size_t)i * cols + 1];
-    const double rz = dim3 ? r[(size_t)i * cols + 2] : 0.0;
-    if (dim3 && (rz - z) > cutoff) return;
-    const double res = x[1] - x[0];
-    const int xa = (int)floor((rx - cutoff - xmin) / res);
-    const int ya = (int)floor((ry - cutoff - ymin) / res);
-    const int xb = (int)floor((rx + cutoff - xmin) / res);
-    const int yb = (int)floor((ry + cutoff - ymin) / res);
-    const double wgt = a[i] * m[i] / rho[i];
-    const double hi = h[i], c2 = cutoff * cutoff;
-    for (int ypx = ya; ypx < yb; ++ypx) {
-        int yy = ypx;
-        if (yy >= ny) yy -= ny;
-        if (yy < 0) yy += ny;
-        if (yy < 0 || yy >= ny) continue;  // boxes wider than the grid
-        for (int xpx = xa; xpx < xb; ++xpx) {
-            int xx = xpx;
-            if (xx >= nx) xx -= nx;
-            if (xx < 0) xx += nx;
-            if (xx < 0 || xx >= nx) continue;
-            double dx, dy, dz = 0.0;
-            if (dim3) {
-                dx = rx - x[xx];
-                dy = ry - y[yy];
-                dz = rz - z;
-            } else {
-                dx = rx - x[xx];
-                dy = y[yy] - ry;
+struct SplatArgs {
+    int n, cols, nx, ny, dim3, per;   // per: particles of a warp
+    const double *r, *m, *rho, *a, *h, *x, *y;
+    double z, xmin, xmax, ymin, ymax, cutoff;
+    double *Z;
+};
+
+// A particle's pixel box and weights, on the lane that prepares it.
+struct Splat {
+    double rx, ry, dz2, coef, inv_h;
+    int xa, ya, w, hgt;   // first pixel, box extents (0: nothing to draw)
+};
+
+__device__ __forceinline__ Splat splat_prepare(const SplatArgs &A, int i, double res) {
+    Splat s;
+    const double *r = A.r + (size_t)i * A.cols;
+    s.rx = r[0];
+    s.ry = r[1];
+    const double dz = A.dim3 ? r[2] - A.z : 0.0;
+    s.dz2 = dz * dz;
+    s.xa = (int)floor((s.rx - A.cutoff - A.xmin) / res);
+    s.ya = (int)floor((s.ry - A.cutoff - A.ymin) / res);
+    const int xb = (int)floor((s.rx + A.cutoff - A.xmin) / res);
+    const int yb = (int)floor((s.ry + A.cutoff - A.ymin) / res);
+    // indices wrap once: of a box wider than the grid's three images only the
+    // pixels in range are drawn, so it may end there
+    s.xa = max(s.xa, -A.nx);
+    s.ya = max(s.ya, -A.ny);
+    s.w = max(0, min(xb, 2 * A.nx) - s.xa);
+    s.hgt = max(0, min(yb, 2 * A.ny) - s.ya);
+    if (A.dim3 && dz > A.cutoff) s.w = 0;
+    const double pi = 3.14159265358979323846;
+    const double wgt = A.a[i] * A.m[i] / A.rho[i], h = A.h[i];
+    // a smoothing length that is not positive draws zeros (wgt 0)
+    s.inv_h = h > 0.0 ? 1.0 / h : 0.0;
+    s.coef = wgt * (h > 0.0 ? (A.dim3 ? 105.0 / (pi * 16.0 * (h * h * h)) : 5.0 / (pi * h * h))
+                            : 0.0);
+    return s;
+}
+
+__device__ __forceinline__ int wrap_once(int k, int n) {
+    if (k >= n) k -= n;
+    if (k < 0) k += n;
+    return k;
+}
+
+// d less or greater than L/2, decided by the high words but for ties: a compare
+// costs the FP64 pipe as much as an addition
+__device__ __forceinline__ double fast_image(double d, double L) {
+    const double half = 0.5 * L;
+    if ((__double2hiint(d) & 0x7fffffff) < __double2hiint(half)) return d;
+    return min_image(d, L);
+}
+__device__ __forceinline__ bool fast_less(double x, double y) {   // squares
+    const int a = __double2hiint(x) & 0x7fffffff, b = __double2hiint(y);
+    return a != b ? a < b : x < y;
+}
+
+// Pixels found and not yet drawn.
+struct SplatQueue {
+    double rsq[64];
+    int2 px[64];
+    unsigned char k[64];   // the particle, as the lane that prepared it
+};
+
+// Draws one found pixel per lane (the first `n` of the queue).
+__device__ __forceinline__ void splat_draw(const SplatArgs &A, const SplatQueue &q, int n,
+                                           const Splat &mine) {
+    const int lane = threadIdx.x & 31, k = lane < n ? q.k[lane] : 0;
+    const double coef = __shfl_sync(0xffffffffu, mine.coef, k);
+    const double inv_h = __shfl_sync(0xffffffffu, mine.inv_h, k);
+    if (lane >= n) return;
+    // Lucy: q (1 + 3 s/h) (1 - s/h)^3
+    double ih, t = fma(-sph::tile_sqrt(q.rsq[lane], &ih), inv_h, 1.0);
+    if (__double2hiint(t) < 0) t = 0.0;
+    const int2 px = q.px[lane];
+    atomicAdd(&A.Z[(size_t)px.x * A.ny + px.y], coef * (t * t * t) * fma(-3.0, t, 4.0));
+}
+
+// A warp per `per` particles: each lane prepares one (the divisions of a
+// particle's box and weight are FP64 work that costs a warp the same for one
+// lane), then the warp goes through them, a lane per pixel of the box; the pixels
+// inside the cutoff (78% of a box) are queued across particles and drawn 32 at a
+// time, so that the drawing, 13 FP64 operations a pixel and what bounds the
+// kernel, has no idle lanes.  One thread per particle took 1.29 ms for 100,172
+// particles on 635 x 633 pixels (94 pixels each), a lane per pixel without the
+// queue 0.74 ms, this form 0.47 ms.
+__global__ void __launch_bounds__(128) k_splat(const SplatArgs A) {
+    __shared__ SplatQueue queues[4];
+    SplatQueue &q = queues[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int first = (blockIdx.x * 4 + (threadIdx.x >> 5)) * A.per;
+    if (first >= A.n) return;
+    const double res = A.x[1] - A.x[0], c2 = A.cutoff * A.cutoff;
+    const int count = min(A.per, A.n - first);
+    const Splat mine = splat_prepare(A, min(first + lane, A.n - 1), res);
+    int queued = 0;
+    for (int k = 0; k < count; ++k) {
+        const int w = __shfl_sync(0xffffffffu, mine.w, k);
+        const int hgt = __shfl_sync(0xffffffffu, mine.hgt, k);
+        if (w == 0 || hgt == 0) continue;
+        const int xa = __shfl_sync(0xffffffffu, mine.xa, k);
+        const int ya = __shfl_sync(0xffffffffu, mine.ya, k);
+        const double rx = __shfl_sync(0xffffffffu, mine.rx, k);
+        const double ry = __shfl_sync(0xffffffffu, mine.ry, k);
+        const double dz2 = __shfl_sync(0xffffffffu, mine.dz2, k);
+        // boxes of at most 32 columns and rows (the rule): each lane holds the
+        // squared distance of one column and one row
+        const bool small = w <= 32 && hgt <= 32;
+        double dx2 = 0.0, dy2 = 0.0;
+        if (small) {
+            const int xx = wrap_once(xa + lane, A.nx), yy = wrap_once(ya + lane, A.ny);
+            const double dx = fast_image(rx - A.x[min(max(xx, 0), A.nx - 1)], A.xmax);
+            const double dy = fast_image(A.y[min(max(yy, 0), A.ny - 1)] - ry, A.ymax);
+            dx2 = dx * dx;
+            dy2 = fma(dy, dy, dz2);
+        }
+        const long long pixels = (long long)w * hgt;
+        int col = lane % w, row = lane / w;
+        const int dc = 32 % w, dr = 32 / w;
+        for (long long p = lane; p - lane < pixels; p += 32) {
+            const int xx = wrap_once(xa + col, A.nx), yy = wrap_once(ya + row, A.ny);
+            const bool ok = p < pixels && xx >= 0 && xx < A.nx && yy >= 0 && yy < A.ny;
+            double rsq = 0.0;
+            if (small) {
+                rsq = __shfl_sync(0xffffffffu, dx2, col) + __shfl_sync(0xffffffffu, dy2, row & 31);
+            } else if (ok) {
+                const double dx = fast_image(rx - A.x[xx], A.xmax);
+                const double dy = fast_image(A.y[yy] - ry, A.ymax);
+                rsq = fma(dx, dx, fma(dy, dy, dz2));
             }
-            dx = min_image(dx, xmax);
-            dy = min_image(dy, ymax);
-            double rsq = dx * dx + dy * dy + dz * dz;
-            if (rsq < c2) atomicAdd(&Z[(size_t)xx * ny + yy], wgt * lucy_w(sqrt(rsq), hi, dim3));
+            const bool in = ok && fast_less(rsq, c2);
+            const unsigned mask = __ballot_sync(0xffffffffu, in);
+            if (in) {
+                const int at = queued + __popc(mask & ((1u << lane) - 1u));
+                q.rsq[at] = rsq;
+                q.px[at] = make_int2(xx, yy);
+                q.k[at] = (unsigned char)k;
+            }
+            queued += __popc(mask);
+            if (queued >= 32) {
+                __syncwarp();
+                splat_draw(A, q, 32, mine);
+                queued -= 32;
+                // the rest moves to the front
+                const bool keep = lane < queued;
+                const double r2 = q.rsq[32 + lane];
+                const int2 px = q.px[32 + lane];
+                const unsigned char kk = q.k[32 + lane];
+                __syncwarp();
+                if (keep) {
+                    q.rsq[lane] = r2;
+                    q.px[lane] = px;
+                    q.k[lane] = kk;
+                }
+                __syncwarp();
+            }
+            col += dc;
+            row += dr;
+            if (col >= w) {
+                col -= w;
+                ++row;
+            }
         }
     }
+    __syncwarp();
+    splat_draw(A, q, queued, mine);
 }
 
 }  // namespace
@@ -121,10 +236,17 @@ extern "C" int sph_splash_map(int32_t mode, int64_t n, const double *r, int32_t 
         da = rho;
     }
     cudaMemsetAsync(dZ, 0, sizeof(double) * npix, st);
-    if (n > 0)
-        k_splat<<<(int)((n + 127) / 128), 128, 0, st>>>(
-            (int)n, dr, r_cols, dm, drho, da, dh, nx, ny, dx, dy, z, bounds[0], bounds[1],
-            bounds[2], bounds[3], cutoff, mode == 3 ? 1 : 0, dZ);
+    if (n > 0) {
+        // enough warps for eight on every SM, at most 32 particles each
+        const int sms = sph::device_sms();
+        const int per = (int)std::min<int64_t>(32, std::max<int64_t>(1, n / (8 * sms)));
+        const SplatArgs A = {(int)n,    r_cols,    nx,        ny,        mode == 3 ? 1 : 0,
+                             per,       dr,        dm,        drho,      da,
+                             dh,        dx,        dy,        z,         bounds[0],
+                             bounds[1], bounds[2], bounds[3], cutoff,    dZ};
+        const int64_t warps = (n + per - 1) / per;
+        k_splat<<<(int)((warps + 3) / 4), 128, 0, st>>>(A);
+    }
     int status = SPH_OK;
     if (mem == SPH_HOST) {
         if (cudaMemcpyAsync(Z, dZ, sizeof(double) * npix, cudaMemcpyDeviceToHost, st) !=

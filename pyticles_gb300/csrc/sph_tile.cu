@@ -49,26 +49,6 @@ constexpr int kTileCap = 256;
 using TileSlot = unsigned char;
 constexpr int kTileThreads = 32 * kTileRounds;
 
-// ---- FP64 helpers: the reciprocal and square root of the pair bodies, from
-// the hardware's approximations (rcp.approx, rsqrt.approx) by Newton and
-// Goldschmidt iterations (Markstein, Software Division and Square Root Using
-// Goldschmidt's Algorithms, 2004), without the range checks and branches that
-// the general functions need: arguments here are positive and normal ----
-
-// sqrt(x); *ih receives 1/(2 sqrt(x)) to about 2^-40.
-__device__ __forceinline__ double tile_sqrt(double x, double *ih) {
-    // coincident particles: r = 1e-140 instead of 0 (d = 0, so no term sees it)
-    if (__double2hiint(x) < 0x05D00000) x = 1e-280;
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double g = x * y, h = 0.5 * y;
-    const double r = fma(-h, g, 0.5);
-    g = fma(g, r, g);
-    *ih = fma(h, r, h);
-    const double d = fma(-g, g, x);
-    return fma(d, h, g);
-}
-
 // 1/r from r and ih = 1/(2r) to about 2^-40.
 __device__ __forceinline__ double tile_inv(double r, double ih) {
     const double e = fma(-ih, r, 0.5);
