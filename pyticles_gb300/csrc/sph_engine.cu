@@ -155,6 +155,8 @@ struct sph_engine {
     int graph_steps = 0;
     bool graph_launched = false;   // its event slots hold a launch's profile
     bool props_valid = false;
+    void *xbuf = nullptr;          // workspace of the pair export
+    size_t xbuf_size = 0;
 };
 
 namespace {
@@ -1285,6 +1287,24 @@ int write_state_range(sph_engine *e, int off, int64_t n, const double *r, const 
     return SPH_OK;
 }
 
+// Room of `bytes` in the pair export's workspace, keeping its first `keep` bytes.
+// The engine keeps the workspace between calls up to kExportKeep bytes.
+constexpr size_t kExportKeep = size_t(256) << 20;
+int export_room(sph_engine *e, size_t bytes, size_t keep = 0) {
+    if (bytes <= e->xbuf_size) return SPH_OK;
+    const size_t want = std::max(bytes, std::min(bytes + bytes / 4, kExportKeep));
+    char *p = nullptr;
+    TRY(dalloc(&p, want));
+    if (keep) {
+        CK(cudaMemcpyAsync(p, e->xbuf, keep, cudaMemcpyDeviceToDevice, e->stream));
+        CK(cudaStreamSynchronize(e->stream));
+    }
+    cudaFree(e->xbuf);
+    e->xbuf = p;
+    e->xbuf_size = want;
+    return SPH_OK;
+}
+
 int copy_out(sph_engine *e, double *dst, size_t count, int mem, double *dev_src) {
     if (mem == SPH_DEVICE) return SPH_OK;  // written in place
     CK(cudaMemcpyAsync(dst, dev_src, sizeof(double) * count, cudaMemcpyDeviceToHost, e->stream));
@@ -1418,7 +1438,7 @@ void free_all(sph_engine *e) {
                     e->pk_vel[0], e->pk_vel[1], e->pk_f, e->pk_q, e->pk_fv, e->ue, e->rho, e->rho_l,
                     e->temp, e->pres, e->pco, e->rho0, e->pres0, e->pco0, e->udot, e->f0u,
                     e->acc_u, e->stage_buf, e->sims_d, e->t_scale, e->tsum_part, e->steps_d,
-                    e->pair_count, e->err, e->err_any, e->rebin_gate, e->restage_far, e->n_items,
+                    e->pair_count, e->err, e->err_any, e->rebin_gate, e->restage_far, e->n_items, e->xbuf,
                     e->bin_count,
                     e->chunk_sim, e->chunk_start,
                     e->chunk_len, e->cell_xyz};
@@ -1893,8 +1913,8 @@ int sph_sim_export_pairs(sph_engine *e, int32_t id, int64_t cap, int64_t *iap, d
     const Sim &S = e->sims[id];
     View v = make_view(e);
     stage_view(e, v, 0);
-    long long *rows = nullptr;
-    TRY(dalloc(&rows, (size_t)S.n + 1));
+    TRY(export_room(e, sizeof(long long) * ((size_t)S.n + 1)));
+    long long *rows = (long long *)e->xbuf;
     CK(cudaMemsetAsync(rows, 0, sizeof(long long) * (S.n + 1), st));
     launch_pair_rows(v, e->precision, S.part_off, (int)S.n, rows, st);
     launch_scan64(rows, (int)S.n, st);
@@ -1902,52 +1922,42 @@ int sph_sim_export_pairs(sph_engine *e, int32_t id, int64_t cap, int64_t *iap, d
     CK(cudaMemcpyAsync(&total, rows + S.n, sizeof(total), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     *nip = total;
-    if (total > cap) {
-        cudaFree(rows);
-        return SPH_ECAPACITY;
+    if (total > cap) return SPH_ECAPACITY;
+    if (total == 0 || !(iap || drij || rsq || dv)) return SPH_OK;
+    // the pairs found, in no order, and with host arrays a device copy of each
+    const bool host = mem == SPH_HOST;
+    const size_t np = (size_t)total, d = (size_t)e->dim;
+    const size_t at_found = sizeof(long long) * ((size_t)S.n + 1);
+    size_t at = at_found + sizeof(int2) * np;
+    auto take = [&](const void *want, size_t bytes) {
+        const size_t here = at;
+        if (want && host) at += bytes;
+        return here;
+    };
+    const size_t at_iap = take(iap, 16 * np), at_drij = take(drij, 8 * np * d);
+    const size_t at_rsq = take(rsq, 8 * np), at_dv = take(dv, 8 * np * d);
+    int status = export_room(e, at, at_found);
+    if (status != SPH_OK) return status;
+    char *x = (char *)e->xbuf;
+    auto place = [&](void *want, size_t here) {
+        return !want ? nullptr : (host ? (void *)(x + here) : want);
+    };
+    launch_pair_write(v, e->precision, S.part_off, (int)S.n, (const long long *)x,
+                      (int2 *)(x + at_found), (long long *)place(iap, at_iap),
+                      (double *)place(drij, at_drij), (double *)place(rsq, at_rsq),
+                      (double *)place(dv, at_dv), st);
+    if (host) {
+        if (iap) CK(cudaMemcpyAsync(iap, x + at_iap, 16 * np, cudaMemcpyDeviceToHost, st));
+        if (drij) CK(cudaMemcpyAsync(drij, x + at_drij, 8 * np * d, cudaMemcpyDeviceToHost, st));
+        if (rsq) CK(cudaMemcpyAsync(rsq, x + at_rsq, 8 * np, cudaMemcpyDeviceToHost, st));
+        if (dv) CK(cudaMemcpyAsync(dv, x + at_dv, 8 * np * d, cudaMemcpyDeviceToHost, st));
     }
-    if (total > 0 && (iap || drij || rsq || dv)) {
-        long long *d_iap = nullptr;
-        double *d_drij = nullptr, *d_rsq = nullptr, *d_dv = nullptr;
-        bool host = mem == SPH_HOST;
-        int st1 = SPH_OK;
-        if (host || !iap) st1 = dalloc(&d_iap, (size_t)total * 2);
-        else d_iap = (long long *)iap;
-        if (st1 == SPH_OK && drij) {
-            if (host) st1 = dalloc(&d_drij, (size_t)total * e->dim);
-            else d_drij = drij;
-        }
-        if (st1 == SPH_OK && rsq) {
-            if (host) st1 = dalloc(&d_rsq, (size_t)total);
-            else d_rsq = rsq;
-        }
-        if (st1 == SPH_OK && dv) {
-            if (host) st1 = dalloc(&d_dv, (size_t)total * e->dim);
-            else d_dv = dv;
-        }
-        if (st1 == SPH_OK) {
-            launch_pair_write(v, e->precision, S.part_off, (int)S.n, rows, d_iap, d_drij, d_rsq,
-                              d_dv, st);
-            if (host) {
-                if (iap) cudaMemcpyAsync(iap, d_iap, sizeof(long long) * total * 2, cudaMemcpyDeviceToHost, st);
-                if (drij) cudaMemcpyAsync(drij, d_drij, sizeof(double) * total * e->dim, cudaMemcpyDeviceToHost, st);
-                if (rsq) cudaMemcpyAsync(rsq, d_rsq, sizeof(double) * total, cudaMemcpyDeviceToHost, st);
-                if (dv) cudaMemcpyAsync(dv, d_dv, sizeof(double) * total * e->dim, cudaMemcpyDeviceToHost, st);
-            }
-            cudaStreamSynchronize(st);
-        }
-        if (host || !iap) cudaFree(d_iap);
-        if (host) {
-            cudaFree(d_drij);
-            cudaFree(d_rsq);
-            cudaFree(d_dv);
-        }
-        if (st1 != SPH_OK) {
-            cudaFree(rows);
-            return st1;
-        }
+    CK(cudaStreamSynchronize(st));
+    if (e->xbuf_size > kExportKeep) {
+        cudaFree(e->xbuf);
+        e->xbuf = nullptr;
+        e->xbuf_size = 0;
     }
-    cudaFree(rows);
     CK(cudaGetLastError());
     return SPH_OK;
 }

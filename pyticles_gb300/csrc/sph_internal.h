@@ -379,9 +379,10 @@ void tile_force(const View &v, int kernel, int vh, int integ, int stage, int mod
 int device_sms();   // SMs of the current device
 void launch_pair_rows(const View &v, int precision, int sim_off, int n, long long *row_count,
                       cudaStream_t s);
+// found: scratch of one entry per pair; iap, drij, rsq and dv may each be null
 void launch_pair_write(const View &v, int precision, int sim_off, int n,
-                       const long long *row_start, long long *iap, double *drij, double *rsq,
-                       double *dv, cudaStream_t s);
+                       const long long *row_start, int2 *found, long long *iap, double *drij,
+                       double *rsq, double *dv, cudaStream_t s);
 void launch_scan64(long long *data, int n, cudaStream_t s);
 
 }  // namespace sph

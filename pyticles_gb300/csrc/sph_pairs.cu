@@ -355,57 +355,71 @@ void launch_tsum(const View &v, int precision, int nsims, cudaStream_t s) {
 
 // ---- pair-set export (VerletList.build + NeighbourList.separations
 // attributes): the same pair iteration, rows keyed by original index ----
-template <typename R, int D>
-__global__ void k_pair_rows(View v, int off, int n, long long *row_count) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    int i = off + k;
+//
+// A warp per particle, a lane per window cell.  The order of a row is that of
+// its partners' original indices: the warp files the partners as it finds them
+// and every partner's place is the number of smaller indices in the row, counted
+// by its lane from the row in L1.  16,002 particles with 58 partners each: rows
+// counted in 148 us and written in 190; one thread per particle, inserting each
+// partner into the row in global memory, took 2.5 and 6.4 ms (in cells 2.5 times
+// as wide, which the neighbour list then asked for).
+template <typename R, int D, typename F>
+__device__ __forceinline__ void export_pairs(const View &v, int i, F found) {
     const SimDev &S = v.sims[v.b_sim[i]];
     using T4 = typename V4<R>::T;
     const T4 *__restrict__ P = (const T4 *)v.pk_pos_in;
     PairFrame<R, D> fr;
     fr.init(S);
     const int idi = v.b_id[i];
-    long long c = 0;
-    for_pairs<R, D>(
-        v, S, fr, P, i, P[i], [&](int j, const T4 &, const R *, R, auto) {
-            if (v.b_id[j] > idi) ++c;
+    for_pairs_lanes<R, D, 32, true>(
+        v, S, fr, P, i, P[i], true,
+        [&](int j, const T4 &, const R *, R, auto) {
+            const int idj = v.b_id[j];
+            if (idj > idi) found(idj, j);
         },
-        [] {});
-    row_count[idi] = c;
+        [](unsigned) {});
+}
+
+constexpr int kExportWarps = 4;
+
+template <typename R, int D>
+__global__ void __launch_bounds__(32 * kExportWarps) k_pair_rows(View v, int off, int n,
+                                                                 long long *row_count) {
+    const int k = blockIdx.x * kExportWarps + (threadIdx.x >> 5);
+    if (k >= n) return;
+    int c = 0;
+    export_pairs<R, D>(v, off + k, [&](int, int) { ++c; });
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0) row_count[v.b_id[off + k]] = c;
 }
 
 template <typename R, int D>
-__global__ void k_pair_write(View v, int off, int n, const long long *row_start, long long *iap,
-                             double *drij, double *rsq, double *dv) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * kExportWarps)
+    k_pair_write(View v, int off, int n, const long long *row_start, int2 *found,
+                 long long *iap, double *drij, double *rsq, double *dv) {
+    __shared__ int filed[kExportWarps];
+    const int k = blockIdx.x * kExportWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (k >= n) return;
-    int i = off + k;
-    const SimDev &S = v.sims[v.b_sim[i]];
-    using T4 = typename V4<R>::T;
-    const T4 *__restrict__ P = (const T4 *)v.pk_pos_in;
-    PairFrame<R, D> fr;
-    fr.init(S);
-    const int idi = v.b_id[i];
+    int &m = filed[threadIdx.x >> 5];
+    const int i = off + k, idi = v.b_id[i];
     const long long base = row_start[idi];
-    long long m = 0;
-    for_pairs<R, D>(v, S, fr, P, i, P[i], [&](int j, const T4 &, const R *, R, auto) {
-        const int idj = v.b_id[j];
-        if (idj < idi) return;
-        // insertion into the row, ordered by j's original index
-        long long p = base + m;
-        while (p > base && iap[2 * (p - 1) + 1] > idj) {
-            iap[2 * p] = iap[2 * (p - 1)];
-            iap[2 * p + 1] = iap[2 * (p - 1) + 1];
-            if (rsq) rsq[p] = rsq[p - 1];
-            if (drij)
-                for (int a = 0; a < D; ++a) drij[p * D + a] = drij[(p - 1) * D + a];
-            if (dv)
-                for (int a = 0; a < D; ++a) dv[p * D + a] = dv[(p - 1) * D + a];
-            --p;
+    int2 *row = found + base;
+    if (lane == 0) m = 0;
+    __syncwarp();
+    export_pairs<R, D>(v, i, [&](int idj, int j) { row[atomicAdd(&m, 1)] = make_int2(idj, j); });
+    __syncwarp();
+    const SimDev &S = v.sims[v.b_sim[i]];
+    const int total = m;
+    for (int e = lane; e < total; e += 32) {
+        const int2 mine = row[e];
+        int rank = 0;
+        for (int t = 0; t < total; ++t) rank += row[t].x < mine.x ? 1 : 0;
+        const long long p = base + rank;
+        const int j = mine.y;
+        if (iap) {
+            iap[2 * p] = idi;
+            iap[2 * p + 1] = mine.x;
         }
-        iap[2 * p] = idi;
-        iap[2 * p + 1] = idj;
         double r2 = 0.0;
         for (int a = 0; a < D; ++a) {
             double d = __dsub_rn(v.xe_in[a][j], v.xe_in[a][i]);
@@ -416,61 +430,73 @@ __global__ void k_pair_write(View v, int off, int n, const long long *row_start,
             if (dv) dv[p * D + a] = __dsub_rn(v.ve_in[a][j], v.ve_in[a][i]);
         }
         if (rsq) rsq[p] = r2;
-        ++m;
-    }, [] {});
+    }
 }
+
+#define SPH_EXPORT(FN, ...)                                                              \
+    do {                                                                                 \
+        const int nb = (n + kExportWarps - 1) / kExportWarps, nt = 32 * kExportWarps;    \
+        if (precision == SPH_MIXED) {                                                    \
+            if (v.dim == 2) FN<float, 2><<<nb, nt, 0, s>>>(v, sim_off, n, __VA_ARGS__);  \
+            else FN<float, 3><<<nb, nt, 0, s>>>(v, sim_off, n, __VA_ARGS__);             \
+        } else {                                                                         \
+            if (v.dim == 2) FN<double, 2><<<nb, nt, 0, s>>>(v, sim_off, n, __VA_ARGS__); \
+            else FN<double, 3><<<nb, nt, 0, s>>>(v, sim_off, n, __VA_ARGS__);            \
+        }                                                                                \
+    } while (0)
 
 void launch_pair_rows(const View &v, int precision, int sim_off, int n, long long *row_count,
                       cudaStream_t s) {
     if (n <= 0) return;
-    int nb = (n + 127) / 128;
-    if (precision == SPH_MIXED) {
-        if (v.dim == 2) k_pair_rows<float, 2><<<nb, 128, 0, s>>>(v, sim_off, n, row_count);
-        else k_pair_rows<float, 3><<<nb, 128, 0, s>>>(v, sim_off, n, row_count);
-    } else {
-        if (v.dim == 2) k_pair_rows<double, 2><<<nb, 128, 0, s>>>(v, sim_off, n, row_count);
-        else k_pair_rows<double, 3><<<nb, 128, 0, s>>>(v, sim_off, n, row_count);
-    }
+    SPH_EXPORT(k_pair_rows, row_count);
 }
 
 void launch_pair_write(const View &v, int precision, int sim_off, int n,
-                       const long long *row_start, long long *iap, double *drij, double *rsq,
-                       double *dv, cudaStream_t s) {
+                       const long long *row_start, int2 *found, long long *iap, double *drij,
+                       double *rsq, double *dv, cudaStream_t s) {
     if (n <= 0) return;
-    int nb = (n + 127) / 128;
-#define SPH_PW(R_, D_) \
-    k_pair_write<R_, D_><<<nb, 128, 0, s>>>(v, sim_off, n, row_start, iap, drij, rsq, dv)
-    if (precision == SPH_MIXED) {
-        if (v.dim == 2) SPH_PW(float, 2);
-        else SPH_PW(float, 3);
-    } else {
-        if (v.dim == 2) SPH_PW(double, 2);
-        else SPH_PW(double, 3);
-    }
-#undef SPH_PW
+    SPH_EXPORT(k_pair_write, row_start, found, iap, drij, rsq, dv);
 }
+#undef SPH_EXPORT
 
-// exclusive scan of n+1 int64 entries in place (export path only)
-__global__ void k_scan64(long long *data, int n) {
-    __shared__ long long sh[1024];
-    __shared__ long long carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base <= n; base += 1024) {
-        int i = base + threadIdx.x;
-        long long x = (i <= n) ? data[i] : 0;
-        sh[threadIdx.x] = x;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            long long y = threadIdx.x >= (unsigned)o ? sh[threadIdx.x - o] : 0;
-            __syncthreads();
-            sh[threadIdx.x] += y;
-            __syncthreads();
+// Exclusive scan of n + 1 int64 entries in place (export path only): one block,
+// eight entries a thread and two barriers per 8,192.
+constexpr int kScan64Per = 8;
+__global__ void __launch_bounds__(1024) k_scan64(long long *data, int n) {
+    __shared__ long long warp_sum[2][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    long long carry = 0;
+    for (int base = 0, round = 0; base <= n; base += 1024 * kScan64Per, round ^= 1) {
+        const int i0 = base + threadIdx.x * kScan64Per;
+        long long x[kScan64Per], sum = 0;
+#pragma unroll
+        for (int t = 0; t < kScan64Per; ++t) {
+            x[t] = i0 + t <= n ? data[i0 + t] : 0;
+            sum += x[t];
         }
-        if (i <= n) data[i] = sh[threadIdx.x] - x + carry;
+        long long incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) warp_sum[round][w] = incl;
         __syncthreads();
-        if (threadIdx.x == 1023) carry += sh[1023];
-        __syncthreads();
+        // every warp scans the warps' sums; the other round's are still read
+        long long ws = warp_sum[round][lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long y = __shfl_up_sync(0xffffffffu, ws, o);
+            if (lane >= o) ws += y;
+        }
+        const long long before = __shfl_sync(0xffffffffu, ws, w > 0 ? w - 1 : 0);
+        long long at = carry + (w > 0 ? before : 0) + incl - sum;
+#pragma unroll
+        for (int t = 0; t < kScan64Per; ++t) {
+            if (i0 + t <= n) data[i0 + t] = at;
+            at += x[t];
+        }
+        carry += __shfl_sync(0xffffffffu, ws, 31);
     }
 }
 

@@ -43,8 +43,11 @@ class NeighbourList:
         p = self.particle
         n = p.n
         cutoff, tol = self._cutoff_tol()
+        # the engine never steps: a small dt leaves its cells without room for drift
+        # (with dt = 1 and thermal velocities a window held 6,250 candidates of
+        # 16,002 particles instead of 230)
         prm = _abi.make_params(dim=p.dim, kernel="lucy", box=p.box.extents, h_short=1.0,
-                               h_long=1.0, cutoff=cutoff, tolerance=tol, dt=1.0)
+                               h_long=1.0, cutoff=cutoff, tolerance=tol, dt=1e-9)
         key = (n, p.dim, cutoff, tol, p.box.extents)
         if self._engine is None or self._key != key:
             if self._engine is not None:

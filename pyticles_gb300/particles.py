@@ -299,7 +299,8 @@ class SmoothParticleSystem(ParticleSystem):
         """One evaluation of the rates at the current state on the GPU
         (particles.py:544-567 with SpamComplete.apply)."""
         t = time.time()
-        e = self._ensure_engine(self.dt if self.dt > 0 else 1.0)
+        # before the first step: a dt that leaves the cells without room for drift
+        e = self._ensure_engine(self.dt if self.dt > 0 else 1e-9)
         out = e.derivatives(self._sim)
         e.sync()
         n = self.n

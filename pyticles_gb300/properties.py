@@ -79,7 +79,8 @@ def _densities(p, nl, precision=None):
     cutoff, tol = nl._cutoff_tol()
     prm = _abi.make_params(dim=p.dim, kernel="lucy", box=p.box.extents,
                            h_short=float(p.h[0]), h_long=float(p.hlr[0]), cutoff=cutoff,
-                           tolerance=tol, adash=ADASH, bdash=BDASH, kbdash=KBDASH, dt=1.0)
+                           tolerance=tol, adash=ADASH, bdash=BDASH, kbdash=KBDASH,
+                           dt=1e-9)   # never stepped: cells without room for drift
     precision = precision or getattr(p, "precision", "fp64")
     with Engine(prm, precision, max_particles=max(n, 1)) as e:
         s = e.add(prm, p.r[:n], p.v[:n], p.m[:n], np.zeros(n))
