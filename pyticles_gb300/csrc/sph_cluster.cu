@@ -473,7 +473,7 @@ __device__ __forceinline__ void cl_segment(const View &v, const ClusterSet &c, c
         d[0] = (pj.x + sx) - pi.x;
         d[1] = (pj.y + sy) - pi.y;
         d[2] = (pj.z + sz) - pi.z;
-        const float rsq = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+        const float rsq = fma_(d[2], d[2], fma_(d[1], d[1], d[0] * d[0]));
         if (gi >= 0 && rsq <= x.thr_hi && sj != si &&
             (rsq < x.thr_lo || exact_in_set<3>(v.xe_in, x.S, gi, c.slot_idx[sj]))) {
             body(sj, pj, d, rsq, std::integral_constant<bool, NEAR>{});
@@ -568,10 +568,10 @@ __global__ void __launch_bounds__(kBlock, 6) k_cl_density(const __grid_constant_
             float w, g;
             if constexpr (decltype(near)::value) {
                 kernel_wg<K, float>(ks, dd, &w, &g);
-                rs.add(pj.w * w);
+                rs.madd(pj.w, w);
             }
             kernel_wg<K, float>(kl, dd, &w, &g);
-            rl.add(pj.w * w);
+            rl.madd(pj.w, w);
             ++cnt;
         },
         [&]() {
@@ -642,9 +642,9 @@ __global__ void __launch_bounds__(kBlock, 6) k_cl_heat(const __grid_constant__ V
             const float4 fj = c.cf[sj];   // {p/rho^2, 1/rho, T_hi, T_lo}
             const float dT = (fj.z - fi.z) + (fj.w - fi.w);
             const float f = pj.w * fj.y * dT * g;
-            q[0].add(f * d[0]);
-            q[1].add(f * d[1]);
-            q[2].add(f * d[2]);
+            q[0].madd(f, d[0]);
+            q[1].madd(f, d[1]);
+            q[2].madd(f, d[2]);
         },
         [&]() {
             q[0].flush();
@@ -700,7 +700,8 @@ __global__ void __launch_bounds__(kBlock, ONE ? 4 : 3) k_cl_force(const __grid_c
             const Dist<float> dd = make_dist<float>(rsq);
             const float gl = kernel_g<K, float, true>(kl, dd);
             const float4 fvj = c.cfv[sj];
-            const float dvdx = (fvj.x - fvi.x) * d[0] + (fvj.y - fvi.y) * d[1] + (fvj.z - fvi.z) * d[2];
+            const float dvdx = fma_(fvj.z - fvi.z, d[2],
+                                    fma_(fvj.y - fvi.y, d[1], (fvj.x - fvi.x) * d[0]));
             float gsum = gl, gs = 0.0f;
             if constexpr (NEAR) {
                 gs = kernel_g<K, float, true>(ks, dd);
@@ -708,20 +709,21 @@ __global__ void __launch_bounds__(kBlock, ONE ? 4 : 3) k_cl_force(const __grid_c
                 if (visc && dvdx < 0.0f && gs != 0.0f) {   // gs = 0: ps does not enter
                     const float rhoj = c.crho[sj];
                     const float mu = fdiv<float>(hs * dvdx, rsq + eps_h2);
-                    ps += fdiv<float>(2.0f * (-alpha_c * mu + beta * mu * mu), rhoi + rhoj);
+                    ps += fdiv<float>(2.0f * fma_(beta * mu, mu, -(alpha_c * mu)), rhoi + rhoj);
                 }
-                gsum = ps * gs + gl;
+                gsum = fma_(ps, gs, gl);
             }
-            ax[0].add(gsum * d[0]);
-            ax[1].add(gsum * d[1]);
-            ax[2].add(gsum * d[2]);
-            float du = gsum * dvdx * pj.w;   // twice the term, halved at the end
+            ax[0].madd(gsum, d[0]);
+            ax[1].madd(gsum, d[1]);
+            ax[2].madd(gsum, d[2]);
+            float du = gsum * dvdx;   // twice the term, halved at the end
             if (heat && NEAR) {
                 const float4 qj = c.cq[sj];
-                const float dq = (qi.x + qj.x) * d[0] + (qi.y + qj.y) * d[1] + (qi.z + qj.z) * d[2];
-                du -= 2.0f * dq * gs * pj.w;
+                const float dq = fma_(qi.z + qj.z, d[2],
+                                      fma_(qi.y + qj.y, d[1], (qi.x + qj.x) * d[0]));
+                du = fma_(-2.0f * dq, gs, du);
             }
-            ud.add(du);
+            ud.madd(du, pj.w);
         },
         [&]() {
             ax[0].flush();

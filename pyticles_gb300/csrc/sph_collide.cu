@@ -247,9 +247,14 @@ __device__ void collide_one(const CollideSet &c, int k, Vec3Ref vel, Vec3Ref pos
     }
     if (pk_vel) {
         using T4 = typename V4<R>::T;
-        T4 *P = (T4 *)pk_vel;
-        P[i] = make_v4<R>((R)vi[0], (R)vi[1], D == 3 ? (R)vi[2] : (R)0, (R)0);
-        P[j] = make_v4<R>((R)vj[0], (R)vj[1], D == 3 ? (R)vj[2] : (R)0, (R)0);
+        if constexpr (flat2<R, D>) {   // the velocities of the packed record
+            ((float2 *)pk_vel)[2 * (size_t)i + 1] = make_float2((float)vi[0], (float)vi[1]);
+            ((float2 *)pk_vel)[2 * (size_t)j + 1] = make_float2((float)vj[0], (float)vj[1]);
+        } else {
+            T4 *P = (T4 *)pk_vel;
+            P[i] = make_v4<R>((R)vi[0], (R)vi[1], D == 3 ? (R)vi[2] : (R)0, (R)0);
+            P[j] = make_v4<R>((R)vj[0], (R)vj[1], D == 3 ? (R)vj[2] : (R)0, (R)0);
+        }
     }
     if (push_cut > 0 && drsq < m_(push_cut, push_cut)) {
         // CollisionForce3d: move both particles apart to cutoff + 0.01

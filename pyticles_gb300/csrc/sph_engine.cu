@@ -127,6 +127,7 @@ struct sph_engine {
     int n_tile_sims = 0;           // ... of these, on cell tiles
     int items_max = 0;             // most work items of the cell tiles
     int *n_items = nullptr;
+    int *mass_mixed = nullptr;     // per simulation slot: masses differ
     bool cl_disabled = false;      // cluster lists did not fit: cell passes only
     SimDev one_dev;
     ClusterSet cl = {};            // tuning.pair_scheme = 1 (sph_cluster.cu)
@@ -634,6 +635,10 @@ int alloc_cells(sph_engine *e, int64_t cells) {
     return SPH_OK;
 }
 
+// 2D mixed precision: velocities in the position records, the masses in what
+// are the velocity records otherwise (they do not change between stages).
+bool flat2_layout(const sph_engine *e) { return e->dim == 2 && e->precision == SPH_MIXED; }
+
 View make_view(const sph_engine *e) {
     View v;
     memset(&v, 0, sizeof(v));
@@ -702,6 +707,8 @@ View make_view(const sph_engine *e) {
     v.err = e->err;
     v.err_any = e->err_any;
     v.bin_count = e->bin_count;
+    v.pk_m = flat2_layout(e) ? (float *)e->pk_vel[0] : nullptr;
+    v.mass_mixed = e->mass_mixed;
     v.one_sim = e->one_sim ? 1 : 0;
     if (e->one_sim) v.one = e->one_dev;
     // pair lists once their rows exist (measured)
@@ -948,7 +955,7 @@ void enqueue_collide_apply(sph_engine *e, int s, bool packed, cudaStream_t st) {
     c.np = e->np_b;
     double *const *vel = s == 0 ? e->b_vel : e->ve;
     Vec3Ref vr{{vel[0], vel[1], vel[2]}, 1};
-    launch_collide_apply(c, e->dim, vr, vr, e->b_m, 0.0, packed ? e->pk_vel[0] : nullptr,
+    launch_collide_apply(c, e->dim, vr, vr, e->b_m, 0.0, packed ? (flat2_layout(e) ? e->pk_pos[0] : e->pk_vel[0]) : nullptr,
                          e->precision, e->err, e->err_any, (int)e->sims.size(), st);
 }
 
@@ -1417,6 +1424,8 @@ int alloc_sims(sph_engine *e) {
     TRY(dalloc(&e->err_any, 1));
     TRY(dalloc(&e->rebin_gate, 1));
     TRY(dalloc(&e->n_items, 1));
+    TRY(dalloc(&e->mass_mixed, S));
+    CK(cudaMemset(e->mass_mixed, 0, sizeof(int) * S));
     TRY(dalloc(&e->restage_far, 1));
     TRY(dalloc(&e->bin_count, 1));
     CK(cudaMemset(e->rebin_gate, 0, sizeof(int)));
@@ -1438,7 +1447,7 @@ void free_all(sph_engine *e) {
                     e->pk_vel[0], e->pk_vel[1], e->pk_f, e->pk_q, e->pk_fv, e->ue, e->rho, e->rho_l,
                     e->temp, e->pres, e->pco, e->rho0, e->pres0, e->pco0, e->udot, e->f0u,
                     e->acc_u, e->stage_buf, e->sims_d, e->t_scale, e->tsum_part, e->steps_d,
-                    e->pair_count, e->err, e->err_any, e->rebin_gate, e->restage_far, e->n_items, e->xbuf,
+                    e->pair_count, e->err, e->err_any, e->rebin_gate, e->restage_far, e->n_items, e->mass_mixed, e->xbuf,
                     e->bin_count,
                     e->chunk_sim, e->chunk_start,
                     e->chunk_len, e->cell_xyz};
@@ -1624,7 +1633,8 @@ int sph_sim_add(sph_engine *e, const sph_params *p, int64_t n, const double *r, 
     make_grid(S, e->dim, e->tune.cell_ratio, list_skin_of(e));
     int off = e->a_extent;
     TRY(write_state_range(e, off, n, r, v, m, u, mem));
-    launch_iota_sim(e->a_id + off, e->a_sim + off, id, (int)n, e->stream);
+    launch_iota_sim(e->a_id + off, e->a_sim + off, id, (int)n, e->a_m + off, e->mass_mixed + id,
+                    e->stream);
     CK(cudaMemsetAsync(e->err + id, 0, sizeof(int), e->stream));
     CK(cudaMemsetAsync(e->steps_d + id, 0, sizeof(long long), e->stream));
     CK(cudaStreamSynchronize(e->stream));
@@ -1661,7 +1671,9 @@ int sph_sim_set_state(sph_engine *e, int32_t id, const double *r, const double *
     // A holds the simulation in slot order a_off + k with id[k]; the caller
     // gives original order, so reset ids to identity for the range.
     TRY(write_state_range(e, S.a_off, S.n, r, v, m, u, mem));
-    if (all) launch_iota_sim(e->a_id + S.a_off, e->a_sim + S.a_off, id, (int)S.n, e->stream);
+    if (all)
+        launch_iota_sim(e->a_id + S.a_off, e->a_sim + S.a_off, id, (int)S.n, e->a_m + S.a_off,
+                        e->mass_mixed + id, e->stream);
     // With binning on demand the current cells (and pair lists) are kept
     // when the new state lies within their slack: it goes straight into the
     // simulation's B slots in the current order.  Otherwise the next step

@@ -48,8 +48,7 @@ __device__ __forceinline__ void write_eval_state(const View &v, const SimDev &S,
     skin |= moved > S.vl_eskin2;
     if (skin) set_err(v.err, v.err_any, v.b_sim[i], SPH_ESKIN);
     v.ue_out[i] = u;
-    ((T4 *)v.pk_pos_out)[i] = make_v4<R>(xl[0], xl[1], xl[2], (R)m);
-    ((T4 *)v.pk_vel_out)[i] = make_v4<R>(vv[0], vv[1], vv[2], (R)0);
+    store_packed<R>(v.pk_pos_out, v.pk_vel_out, D == 2, i, xl, vv, (R)m);
 }
 
 // Final state of the step into A (same slot as B), with the teleport wrap.
@@ -96,8 +95,8 @@ __device__ __forceinline__ void write_final_state(const View &v, const SimDev &S
     if (v.reuse) {
         far |= moved > S.vl_gate2;
         v.b_u[i] = u;
-        ((T4 *)v.pk_pos_out)[i] = make_v4<R>(xl[0], xl[1], xl[2], (R)v.b_m[i]);
-        ((T4 *)v.pk_vel_out)[i] = make_v4<R>(vv[0], vv[1], vv[2], (R)0);
+        store_packed<R>(v.pk_pos_out, v.pk_vel_out, D == 2, i, xl, vv,
+                        flat2<R, D> ? (R)0 : (R)v.b_m[i]);
         if (far) *v.rebin_gate = 1;
     }
 }
@@ -201,7 +200,7 @@ __device__ __forceinline__ void integrate_stage(const View &v, const SimDev &S, 
 // simulation, whose constants come from the kernel parameters.
 // Register caps by resident blocks of 256 threads; force of a step, us: a single
 // simulation in 2D (199k particles) 324 / 337 / 294 at 4 / 5 / 6 blocks, in 3D (205k)
-// 2178 / 2248 / 2649 at 3 / 4 / 5; several 623 / 584 / 600 at 3 / 4 / 5.
+// 2178 / 2248 / 2649 at 3 / 4 / 5; 24 simulations in 2D 524 / 531 / 514 at 3 / 4 / 5.
 // LIST: the pair lists (tuning.pair_scheme 2) instead of the cell windows.
 // LANES: lanes per particle (for_pairs_lanes; the same bits).
 template <typename R, int D, int K, int VH, bool ONE, bool LIST = false, int LANES = 1>
@@ -213,6 +212,7 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
     using T4 = typename V4<R>::T;
     const T4 *__restrict__ P = (const T4 *)v.pk_pos_in;
     const T4 *__restrict__ FV = (const T4 *)v.pk_fv;
+    const float2 *__restrict__ FR = (const float2 *)v.pk_fv;   // 2D mixed: {p/rho^2, rho}
     const R *__restrict__ RHO = (const R *)v.rho;
     const T4 *__restrict__ Q = (const T4 *)v.pk_q;
     const int s = v.b_sim[ii];
@@ -228,7 +228,13 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
     const R hs = sc.hs, eps_h2 = sc.eps_h2;
     const R alpha_c = sc.alpha_c, beta = sc.beta;
     // own velocity, p/rho^2 and rho
-    const T4 fvi = FV[ii];
+    T4 fvi;
+    if constexpr (flat2<R, D>) {
+        const T4 p = P[ii];
+        fvi = make_v4<R>(p.z, p.w, FR[ii].x, FR[ii].y);
+    } else {
+        fvi = FV[ii];
+    }
     const R vix = fvi.x, viy = fvi.y, viz = D == 3 ? fvi.z : (R)0;
     const R fsi = D == 2 ? fvi.z : fvi.w;
     const R rhoi = D == 2 ? fvi.w : RHO[ii];
@@ -238,46 +244,6 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
     ax[1].init(0);
     ax[2].init(0);
     ud.init(0);
-    auto body = [&](int j, const T4 &pj, const R *d, R rsq, auto near) {
-        constexpr bool NEAR = decltype(near)::value;
-        const Dist<R> dd = make_dist<R>(rsq);
-        const R gl = kernel_g<K, R, true>(kl, dd);   // -2a grad W_l / r
-        const T4 fvj = FV[j];
-        R dvdx = (fvj.x - vix) * d[0] + (fvj.y - viy) * d[1];
-        if (D == 3) dvdx += (fvj.z - viz) * d[2];
-        // beyond the short support gs = 0: the pressure and viscosity terms
-        // vanish and gsum = gl bit for bit
-        R gsum = gl, gs = (R)0;
-        // the heat record {q/rho^2, rho}: with heat flux in 3D it also
-        // carries the density the viscosity needs
-        T4 qj = make_v4<R>(0, 0, 0, 0);
-        if constexpr (NEAR) {
-            if (heat) qj = Q[j];
-            gs = kernel_g<K, R, true>(ks, dd);
-            R ps = fsi + (D == 2 ? fvj.z : fvj.w);
-            // Monaghan viscosity on approaching pairs within the short
-            // support (beyond it gs = 0, so ps no longer enters gsum and the
-            // warp skips the block when none of its pairs needs it)
-            if (visc && dvdx < (R)0 && gs != (R)0) {
-                const R rhoj = D == 2 ? fvj.w : (heat ? qj.w : RHO[j]);
-                R mu = fdiv<R>(hs * dvdx, rsq + eps_h2);
-                ps += fdiv<R>((R)2 * (-alpha_c * mu + beta * mu * mu), rhoi + rhoj);
-            }
-            gsum = ps * gs + gl;
-        }
-        ax[0].add(gsum * d[0]);
-        ax[1].add(gsum * d[1]);
-        if (D == 3) ax[2].add(gsum * d[2]);
-        // twice the energy-rate term; the sum is halved once at the end
-        // (scaling by 2 is exact, so the bits are those of the halved terms)
-        R du = gsum * dvdx * pj.w;
-        if (heat && NEAR) {
-            R dq = (qi.x + qj.x) * d[0] + (qi.y + qj.y) * d[1];
-            if (D == 3) dq += (qi.z + qj.z) * d[2];
-            du -= (R)2 * dq * gs * pj.w;
-        }
-        ud.add(du);
-    };
     auto cell_done = [&]() {
         ax[0].flush();
         ax[1].flush();
@@ -285,21 +251,76 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
         ud.flush();
     };
     if (LANES == 1 && !active) return;
-    {
+    with_masses<R, D, (LANES > 1)>(v, s, [&](auto same) {
+        const PairMass<R, D, decltype(same)::value> mass(v, ii);
+        auto body = [&](int j, const T4 &pj, const R *d, R rsq, auto near) {
+            constexpr bool NEAR = decltype(near)::value;
+            const Dist<R> dd = make_dist<R>(rsq);
+            const R gl = kernel_g<K, R, true>(kl, dd);   // -2a grad W_l / r
+            T4 fvj;
+            if constexpr (flat2<R, D>) {
+                fvj.x = pj.z;
+                fvj.y = pj.w;
+                if constexpr (NEAR) {
+                    const float2 fr = FR[j];
+                    fvj.z = fr.x;
+                    fvj.w = fr.y;
+                }
+            } else {
+                fvj = FV[j];
+            }
+            const R mj = mass(j, pj);
+            R dvdx = fma_(fvj.y - viy, d[1], (fvj.x - vix) * d[0]);
+            if (D == 3) dvdx = fma_(fvj.z - viz, d[2], dvdx);
+            // beyond the short support gs = 0: the pressure and viscosity terms
+            // vanish and gsum = gl bit for bit
+            R gsum = gl, gs = (R)0;
+            // the heat record {q/rho^2, rho}: with heat flux in 3D it also
+            // carries the density the viscosity needs
+            T4 qj = make_v4<R>(0, 0, 0, 0);
+            if constexpr (NEAR) {
+                if (heat) qj = Q[j];
+                gs = kernel_g<K, R, true>(ks, dd);
+                R ps = fsi + (D == 2 ? fvj.z : fvj.w);
+                // Monaghan viscosity on approaching pairs within the short
+                // support (beyond it gs = 0, so ps no longer enters gsum and the
+                // warp skips the block when none of its pairs needs it)
+                if (visc && dvdx < (R)0 && gs != (R)0) {
+                    const R rhoj = D == 2 ? fvj.w : (heat ? qj.w : RHO[j]);
+                    R mu = fdiv<R>(hs * dvdx, rsq + eps_h2);
+                    ps += fdiv<R>((R)2 * fma_(beta * mu, mu, -(alpha_c * mu)), rhoi + rhoj);
+                }
+                gsum = fma_(ps, gs, gl);
+            }
+            ax[0].madd(gsum, d[0]);
+            ax[1].madd(gsum, d[1]);
+            if (D == 3) ax[2].madd(gsum, d[2]);
+            // twice the energy-rate term; the sum is halved once at the end
+            // (scaling by 2 is exact, so the bits are those of the halved terms)
+            R du = gsum * dvdx;
+            if (heat && NEAR) {
+                R dq = fma_(qi.y + qj.y, d[1], (qi.x + qj.x) * d[0]);
+                if (D == 3) dq = fma_(qi.z + qj.z, d[2], dq);
+                du = fma_((R)-2 * dq, gs, du);
+            }
+            ud.madd(du, mj);
+        };
         PairFrame<R, D> fr;
         fr.init(S);
-        if constexpr (LANES > 1) {
+        if constexpr (LANES > 1)
             for_pairs_lanes<R, D, LANES, false>(v, S, fr, P, ii, P[ii], active, body,
-                                                [&](unsigned mask) {
-                                                    fold_lanes<LANES>(ax[0], mask);
-                                                    fold_lanes<LANES>(ax[1], mask);
-                                                    if (D == 3) fold_lanes<LANES>(ax[2], mask);
-                                                    fold_lanes<LANES>(ud, mask);
-                                                });
-            if (!active || (threadIdx.x & (LANES - 1))) return;
-        } else if constexpr (LIST) for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done, [] {});
-        else for_pairs<R, D, D == 3, false>(v, S, fr, P, i, P[i], body, cell_done);
-    }
+                                                      [&](unsigned mask) {
+                                                          fold_lanes<LANES>(ax[0], mask);
+                                                          fold_lanes<LANES>(ax[1], mask);
+                                                          if (D == 3) fold_lanes<LANES>(ax[2], mask);
+                                                          fold_lanes<LANES>(ud, mask);
+                                                      });
+        else if constexpr (LIST)
+            for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done, [] {});
+        else
+            for_pairs<R, D, D == 3, false>(v, S, fr, P, i, P[i], body, cell_done);
+    });
+    if (LANES > 1 && (!active || (threadIdx.x & (LANES - 1)))) return;
     R vdr[3] = {ax[0].get(), ax[1].get(), ax[2].get()};
     R udr = (R)0.5 * ud.get();
     for (int a = 0; a < D; ++a) ((R *)v.vdot[a])[i] = vdr[a];
@@ -313,7 +334,7 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
 // One thread per particle; PERSIST: the resident blocks of pass_grid walk
 // the particles grid-stride (the same per-particle work, the same bits).
 template <typename R, int D, int K, int VH, bool ONE, bool PERSIST>
-__global__ void __launch_bounds__(256, ONE ? (D == 2 ? 6 : 3) : 4) k_force(const __grid_constant__ View v, int stage,
+__global__ void __launch_bounds__(256, ONE ? (D == 2 ? 6 : 3) : (D == 2 ? 5 : 4)) k_force(const __grid_constant__ View v, int stage,
                                                   int mode, int integ) {
     if constexpr (PERSIST) {
         for (int base = blockIdx.x * blockDim.x; base < v.np; base += gridDim.x * blockDim.x)

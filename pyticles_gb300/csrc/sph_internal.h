@@ -145,11 +145,16 @@ struct View {
     int *cell_xyz;          // global cell -> packed cell coordinates (11/11/10 bits)
     double *org[3];         // B order: FP64 origin of the particle's cell-local frame
     // evaluation (stage s reads *_in, its force pass writes stage s+1's *_out)
-    void *pk_pos_in, *pk_vel_in;     // float4 / double4: {xl, yl, zl, m}, {vx, vy, vz, 0}
+    // packed positions and velocities, float4 / double4: {xl, yl, zl, m} and
+    // {vx, vy, vz, 0}; 2D mixed precision: {xl, yl, vx, vy}, the masses in pk_m
+    void *pk_pos_in, *pk_vel_in;
     void *pk_pos_out, *pk_vel_out;
     void *pk_f, *pk_q;               // {p/rho^2, rho, T_hi, T_lo}, {q/rho^2, rho}
-    void *pk_fv;                     // force-pass view of j: 2D {vx, vy, p/rho^2, rho},
-                                     // 3D {vx, vy, vz, p/rho^2} (rho from `rho`)
+    void *pk_fv;                     // force-pass view of j: 2D {vx, vy, p/rho^2, rho}
+                                     // (mixed precision {p/rho^2, rho}), 3D {vx, vy,
+                                     // vz, p/rho^2} (rho from `rho`)
+    float *pk_m;                     // 2D mixed precision: masses
+    int *mass_mixed;                 // per sim: its particles' masses differ
     double *xe_in[3], *xe_out[3];    // FP64 raw evaluation positions (exact pair test)
     double *ve_in[3], *ve_out[3];    // FP64 evaluation velocities (rdot)
     double *ue_in, *ue_out;          // FP64 evaluation internal energy
@@ -359,7 +364,9 @@ void launch_store_R(double *dst, const void *src, int precision, const int *id, 
 void launch_fill_int(int *dst, int val, int n, cudaStream_t s, const int *gate = nullptr);
 // After a gated binning: clears the gate and counts the binning.
 void launch_rebin_close(int *gate, unsigned long long *bin_count, cudaStream_t s);
-void launch_iota_sim(int *id, int *sim, int sim_id, int n, cudaStream_t s);
+// ids 0 .. n - 1 of simulation sim_id; *mixed is raised if the masses m differ
+void launch_iota_sim(int *id, int *sim, int sim_id, int n, const double *m, int *mixed,
+                     cudaStream_t s);
 
 // ---- launch wrappers (sph_pairs.cu) ----
 // stage: evaluation index within the step; nstage: evaluations per step;

@@ -196,6 +196,8 @@ extern "C" int sph_derivatives_noalloc(const sph_params *p, int32_t precision, i
     w.t_scale = c.take<double>(1);
     w.steps = c.take<long long>(1);
     w.n_items = c.take<int>(1);
+    w.mass_mixed = c.take<int>(1);
+    if (dim == 2 && precision == SPH_MIXED) w.pk_m = (float *)w.pk_vel_in;
     w.item_cell = w.rank;
     w.item_round = w.cell_of;
     w.items_max = (int)n;
@@ -222,7 +224,7 @@ extern "C" int sph_derivatives_noalloc(const sph_params *p, int32_t precision, i
     launch_load_aos(w.a_vel, v, (int)n, dim, st);
     NA_CK(cudaMemcpyAsync(w.a_m, m, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
     NA_CK(cudaMemcpyAsync(w.a_u, u, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
-    launch_iota_sim(w.a_id, w.a_sim, 0, (int)n, st);
+    launch_iota_sim(w.a_id, w.a_sim, 0, (int)n, w.a_m, w.mass_mixed, st);
 
     // the engine's passes: counting sort, density, heat, force (no state update)
     launch_bin(w, (int)n, st);

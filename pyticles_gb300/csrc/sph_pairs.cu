@@ -37,34 +37,33 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
     rs.init((R)0);
     rl.init((R)0);
     unsigned cnt = 0;
-    auto body = [&](int j, const T4 &pj, const R *d, R rsq, auto near) {
-        const Dist<R> dd = plain_dist<R>(rsq);
-        R w, g;
-        if constexpr (decltype(near)::value) {
-            kernel_wg<K, R>(ks, dd, &w, &g);
-            rs.add(pj.w * w);
-        }
-        kernel_wg<K, R>(kl, dd, &w, &g);
-        rl.add(pj.w * w);
-        if (!LIST) ++cnt;
-    };
     auto cell_done = [&]() {
         rs.flush();
         rl.flush();
     };
     if (LANES == 1 && !active) return;
-    {
+    with_masses<R, D, (LANES > 1)>(v, s, [&](auto same) {
+        const PairMass<R, D, decltype(same)::value> mass(v, ii);
+        auto body = [&](int j, const T4 &pj, const R *d, R rsq, auto near) {
+            const Dist<R> dd = plain_dist<R>(rsq);
+            const R mj = mass(j, pj);
+            R w, g;
+            if constexpr (decltype(near)::value) {
+                kernel_wg<K, R>(ks, dd, &w, &g);
+                rs.madd(mj, w);
+            }
+            kernel_wg<K, R>(kl, dd, &w, &g);
+            rl.madd(mj, w);
+            if (!LIST) ++cnt;
+        };
         PairFrame<R, D> fr;
         fr.init(S);
         if constexpr (LANES > 1) {
             for_pairs_lanes<R, D, LANES, true>(v, S, fr, P, ii, P[ii], active, body,
-                                               [&](unsigned mask) {
-                                                   fold_lanes<LANES>(rs, mask);
-                                                   fold_lanes<LANES>(rl, mask);
-                                               });
-#pragma unroll
-            for (int o = LANES / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-            if (!active || (threadIdx.x & (LANES - 1))) return;
+                                                      [&](unsigned mask) {
+                                                          fold_lanes<LANES>(rs, mask);
+                                                          fold_lanes<LANES>(rl, mask);
+                                                      });
         } else if constexpr (LIST) {
             // the entries of whole groups, less those that are no pairs
             const unsigned c = v.vl_cnt[i];
@@ -73,6 +72,11 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
         } else {
             for_pairs<R, D>(v, S, fr, P, i, P[i], body, cell_done);
         }
+    });
+    if constexpr (LANES > 1) {
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+        if (!active || (threadIdx.x & (LANES - 1))) return;
     }
     density_finish<R, D>(v, S, i, s, stage, rs.get64(), rl.get64(), cnt);
 }
@@ -126,6 +130,7 @@ __device__ __forceinline__ void heat_one(const View &v, int i) {
     }
     KConst<R> ks = make_kconst<R>(S, 0);
     const T4 fi = F[ii];
+    const PairMass<R, D, false> mass(v, ii);
     BAcc<R> q[3];
     q[0].init(0);
     q[1].init(0);
@@ -134,10 +139,10 @@ __device__ __forceinline__ void heat_one(const View &v, int i) {
         R g = kernel_g<K, R, true>(ks, make_dist<R>(rsq));
         T4 fj = F[j];
         R dT = (fj.z - fi.z) + (fj.w - fi.w);
-        R f = pj.w * rrcp<R>(fj.y) * dT * g;
-        q[0].add(f * d[0]);
-        q[1].add(f * d[1]);
-        if (D == 3) q[2].add(f * d[2]);
+        R f = mass(j, pj) * rrcp<R>(fj.y) * dT * g;
+        q[0].madd(f, d[0]);
+        q[1].madd(f, d[1]);
+        if (D == 3) q[2].madd(f, d[2]);
     };
     auto cell_done = [&]() {
         q[0].flush();

@@ -111,8 +111,8 @@ __device__ __forceinline__ bool pair_cell(const View &v, const SimDev &S,
             d[1] = pj.y + oy_;
             d[2] = (D == 3) ? pj.z + oz_ : (R)0;
             if constexpr (decltype(mi)::value) fr.min_image(d);
-            R rsq = d[0] * d[0] + d[1] * d[1];
-            if (D == 3) rsq += d[2] * d[2];
+            R rsq = fma_(d[1], d[1], d[0] * d[0]);
+            if (D == 3) rsq = fma_(d[2], d[2], rsq);
             if (rsq > fr.thr_hi) continue;
             if (rsq >= fr.thr_lo && !exact_in_set<D>(v.xe_in, &S, i, j)) continue;
             body(j, pj, d, rsq, near);
@@ -185,7 +185,7 @@ __device__ __forceinline__ void for_pairs(const View &v, const SimDev &S,
         }
         for (int oy = -w1; oy <= w1; ++oy) {
             R dy = fmaxf_((R)oy * fr.edge[1] - pi.y, fr.ext[1]);
-            R dyz = dy * dy + dz * dz;
+            R dyz = fma_(dz, dz, dy * dy);
             if (dyz > fr.thr_hi) continue;
             int y = c1 + oy;
             y += (y < 0) ? n1 : 0;
@@ -193,12 +193,13 @@ __device__ __forceinline__ void for_pairs(const View &v, const SimDev &S,
             const int row = (z * n1 + y) * n0;
             for (int ox = -w0; ox <= w0; ++ox) {
                 R dx = fmaxf_((R)ox * fr.edge[0] - pi.x, fr.ext[0]);
-                if (dx * dx + dyz > fr.thr_hi) continue;
+                const R dxyz = fma_(dx, dx, dyz);
+                if (dxyz > fr.thr_hi) continue;
                 int x = c0 + ox;
                 x += (x < 0) ? n0 : 0;
                 x -= (x >= n0) ? n0 : 0;
                 if (pair_cell<R, D, PF, SELF>(v, S, fr, P, i, pi, mort, row + x, ox, oy, oz,
-                                              dx * dx + dyz < fr.thr_s, body))
+                                              dxyz < fr.thr_s, body))
                     cell_done();
             }
         }
@@ -235,8 +236,9 @@ __device__ __forceinline__ void for_pairs_lanes(const View &v, const SimDev &S,
             const R dx = fmaxf_((R)ox * fr.edge[0] - pi.x, fr.ext[0]);
             const R dy = fmaxf_((R)oy * fr.edge[1] - pi.y, fr.ext[1]);
             const R dz = D == 3 ? fmaxf_((R)oz * fr.edge[2] - pi.z, fr.ext[2]) : (R)0;
-            const R dyz = dy * dy + dz * dz;
-            if (!(dyz > fr.thr_hi) && !(dx * dx + dyz > fr.thr_hi)) {
+            const R dyz = fma_(dz, dz, dy * dy);
+            const R dxyz = fma_(dx, dx, dyz);
+            if (!(dyz > fr.thr_hi) && !(dxyz > fr.thr_hi)) {
                 int x = c0 + ox, y = c1 + oy, z = D == 3 ? c2 + oz : 0;
                 x += x < 0 ? n0 : 0;
                 x -= x >= n0 ? n0 : 0;
@@ -248,7 +250,7 @@ __device__ __forceinline__ void for_pairs_lanes(const View &v, const SimDev &S,
                 }
                 scanned = pair_cell<R, D, false, SELF>(v, S, fr, P, i, pi, mort,
                                                        (z * n1 + y) * n0 + x, ox, oy, oz,
-                                                       dx * dx + dyz < fr.thr_s, body);
+                                                       dxyz < fr.thr_s, body);
             }
         }
         fold((__ballot_sync(0xffffffffu, scanned) >> (lane & ~(G - 1))) &
@@ -315,11 +317,11 @@ __device__ __forceinline__ void for_list(const View &v, const SimDev &S,
         d[0] = __fmaf_rn(fx, fr.edge_lo[0], __fmaf_rn(fx, fr.edge[0], __fsub_rn(pj.x, pi.x)));
         d[1] = __fmaf_rn(fy, fr.edge_lo[1], __fmaf_rn(fy, fr.edge[1], __fsub_rn(pj.y, pi.y)));
         d[2] = (R)0;
-        R rsq = d[0] * d[0] + d[1] * d[1];
+        R rsq = fma_(d[1], d[1], d[0] * d[0]);
         if (D == 3) {
             const float fz = vl_offset(t >> 6);
             d[2] = __fmaf_rn(fz, fr.edge_lo[2], __fmaf_rn(fz, fr.edge[2], __fsub_rn(pj.z, pi.z)));
-            rsq += d[2] * d[2];
+            rsq = fma_(d[2], d[2], rsq);
         }
         // one branch for the guard band and everything beyond it
         if (rsq >= fr.thr_lo && (rsq > fr.thr_hi || !exact_in_set<D>(v.xe_in, &S, i, j))) {
@@ -426,10 +428,14 @@ __device__ __forceinline__ void density_finish(const View &v, const SimDev &S, i
     // {p/rho^2, rho, T_hi, T_lo}: T as a hi/lo pair so that T_j - T_i in the
     // heat pass does not lose the low bits
     ((T4 *)v.pk_f)[i] = make_v4<R>((R)fs, (R)rho, Th, (R)(T - (double)Th));
-    // what the force pass reads of a neighbour, in one 16-byte load in 2D
-    const T4 vi = ((const T4 *)v.pk_vel_in)[i];
-    ((T4 *)v.pk_fv)[i] = D == 2 ? make_v4<R>(vi.x, vi.y, (R)fs, (R)rho)
-                                : make_v4<R>(vi.x, vi.y, vi.z, (R)fs);
+    // what the force pass reads of a neighbour beside its packed record
+    if constexpr (flat2<R, D>) {
+        ((float2 *)v.pk_fv)[i] = make_float2((float)fs, (float)rho);
+    } else {
+        const T4 vi = ((const T4 *)v.pk_vel_in)[i];
+        ((T4 *)v.pk_fv)[i] = D == 2 ? make_v4<R>(vi.x, vi.y, (R)fs, (R)rho)
+                                    : make_v4<R>(vi.x, vi.y, vi.z, (R)fs);
+    }
     if (!isfinite((R)p) || !isfinite((R)rho) || !isfinite((R)rhol))
         set_err(v.err, v.err_any, s, SPH_ENAN);
     // the pair set of one evaluation: counted at the step's first one only

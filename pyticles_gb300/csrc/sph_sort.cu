@@ -237,9 +237,8 @@ __device__ __forceinline__ void permute_one(const View &v, int j) {
     v.b_m[j] = m;
     v.b_id[j] = v.a_id[k];
     v.b_sim[j] = s;
-    using T4 = typename V4<R>::T;
-    ((T4 *)v.pk_pos_out)[j] = make_v4<R>(xl[0], xl[1], xl[2], (R)m);
-    ((T4 *)v.pk_vel_out)[j] = make_v4<R>(vv[0], vv[1], vv[2], (R)0);
+    store_packed<R>(v.pk_pos_out, v.pk_vel_out, v.pk_m, j, xl, vv, (R)m);
+    if (v.pk_m) v.pk_m[j] = (float)m;
 }
 
 template <typename R>
@@ -287,9 +286,8 @@ __global__ void k_restage(View v, int a_off, int b0, int n, int *far) {
     const double m = v.a_m[a];
     v.b_u[j] = v.a_u[a];
     v.b_m[j] = m;
-    using T4 = typename V4<R>::T;
-    ((T4 *)v.pk_pos_out)[j] = make_v4<R>(xl[0], xl[1], xl[2], (R)m);
-    ((T4 *)v.pk_vel_out)[j] = make_v4<R>(vv[0], vv[1], vv[2], (R)0);
+    store_packed<R>(v.pk_pos_out, v.pk_vel_out, v.pk_m, j, xl, vv, (R)m);
+    if (v.pk_m) v.pk_m[j] = (float)m;
     if (out) *far = 1;
 }
 
@@ -388,17 +386,20 @@ void launch_rebin_close(int *gate, unsigned long long *bin_count, cudaStream_t s
     k_rebin_close<<<1, 1, 0, s>>>(gate, bin_count);
 }
 
-__global__ void k_iota_sim(int *id, int *sim, int sim_id, int n) {
+__global__ void k_iota_sim(int *id, int *sim, int sim_id, int n, const double *m, int *mixed) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         id[i] = i;
         sim[i] = sim_id;
+        if (m[i] != m[0]) *mixed = 1;
     }
 }
 
-void launch_iota_sim(int *id, int *sim, int sim_id, int n, cudaStream_t s) {
+void launch_iota_sim(int *id, int *sim, int sim_id, int n, const double *m, int *mixed,
+                     cudaStream_t s) {
     if (n <= 0) return;
-    k_iota_sim<<<(n + 255) / 256, 256, 0, s>>>(id, sim, sim_id, n);
+    cudaMemsetAsync(mixed, 0, sizeof(int), s);
+    k_iota_sim<<<(n + 255) / 256, 256, 0, s>>>(id, sim, sim_id, n, m, mixed);
 }
 
 }  // namespace sph

@@ -27,6 +27,40 @@ def run(sims, steps):
         return list(st) + [pr[k] for k in KEYS] + [e.last_pair_counts(1)]
 
 
+def test_masses_of_neighbouring_simulations():
+    """Equal and mixed masses side by side in one warp, by lanes, by the walk and
+    by pair lists: each simulation's bits are those of its size alone, and equal
+    masses those of the same masses read one by one."""
+    from pyticles_gb300 import Engine
+    sims = []
+    for k, side in enumerate((3, 4, 3, 5, 17, 4)):
+        prm, r, v, m, u = state(workloads.config_2d, side, 50 + k)
+        if k % 2:
+            m = m * np.random.default_rng(k).uniform(0.5, 1.5, len(m))
+        else:
+            m = m * 1.25
+        sims.append((prm, r, v, m, u))
+    for pick in range(len(sims)):
+        order = [sims[pick]] + sims[:pick] + sims[pick + 1:]
+        for a, b in zip(run(sims[pick:pick + 1], 2), run(order, 2)):
+            assert np.array_equal(a, b), pick
+    # masses that differ in one far particle only: the others' pair terms are
+    # summed from masses read one by one
+    prm, r, v, m, u = state(workloads.config_2d, 40, 9)
+    odd = m.copy()
+    far = int(np.argmax(np.abs(r - 10.0).min(axis=1)))
+    odd[far] = 1.5
+    near = np.hypot(*((r - r[far] + 20) % 40 - 20).T) < 14.0
+    with Engine(prm, "mixed", max_particles=len(r)) as e:
+        s = e.add(prm, r, v, m, u)
+        one = e.derivatives(s)
+        e.set_state(s, r, v, odd, u)
+        two = e.derivatives(s)
+        for k in ("rho", "vdot", "udot"):
+            assert np.array_equal(one[k][~near], two[k][~near]), k
+            assert not np.array_equal(one[k], two[k])
+
+
 # 40961 particles and more run one thread per particle
 @pytest.mark.parametrize("maker,sides,big", [
     (workloads.config_2d, [3, 10, 15, 32, 64, 65, 150], 203),
