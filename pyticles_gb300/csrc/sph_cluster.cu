@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(kBlock, ONE ? 4 : 3) k_cl_force(const __grid_c
                 if (visc && dvdx < 0.0f && gs != 0.0f) {   // gs = 0: ps does not enter
                     const float rhoj = c.crho[sj];
                     const float mu = fdiv<float>(hs * dvdx, rsq + eps_h2);
-                    ps += fdiv<float>(2.0f * fma_(beta * mu, mu, -(alpha_c * mu)), rhoi + rhoj);
+                    ps = add_div<float>(2.0f * fma_(beta * mu, mu, -(alpha_c * mu)), rhoi + rhoj, ps);
                 }
                 gsum = fma_(ps, gs, gl);
             }

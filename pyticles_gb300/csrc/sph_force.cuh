@@ -287,8 +287,8 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
                 // warp skips the block when none of its pairs needs it)
                 if (visc && dvdx < (R)0 && gs != (R)0) {
                     const R rhoj = D == 2 ? fvj.w : (heat ? qj.w : RHO[j]);
-                    R mu = fdiv<R>(hs * dvdx, rsq + eps_h2);
-                    ps += fdiv<R>((R)2 * fma_(beta * mu, mu, -(alpha_c * mu)), rhoi + rhoj);
+                    const R mu = fdiv<R>(hs * dvdx, rsq + eps_h2);
+                    ps = add_div<R>((R)2 * fma_(beta * mu, mu, -(alpha_c * mu)), rhoi + rhoj, ps);
                 }
                 gsum = fma_(ps, gs, gl);
             }
