@@ -253,7 +253,13 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
     if (LANES == 1 && !active) return;
     with_masses<R, D, (LANES > 1)>(v, s, [&](auto same) {
         const PairMass<R, D, decltype(same)::value> mass(v, ii);
-        auto body = [&](int j, const T4 &pj, const R *d, R rsq, auto near) {
+        // loaded: what the pair lists fetch of j beside its position, the velocity
+        // record in 3D (in 2D the position record holds the velocity).  Waiting
+        // for it after the test held the 3D list pass up: 3350 us a launch at
+        // 2M particles, 2920 with the load ahead of the test; the heat record
+        // ahead as well made 2960, two or four entries' records at once 3110 and
+        // 3970 (registers).
+        auto body = [&](int j, const T4 &pj, const R *d, R rsq, auto near, auto... loaded) {
             constexpr bool NEAR = decltype(near)::value;
             const Dist<R> dd = make_dist<R>(rsq);
             const R gl = kernel_g<K, R, true>(kl, dd);   // -2a grad W_l / r
@@ -266,6 +272,8 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
                     fvj.z = fr.x;
                     fvj.w = fr.y;
                 }
+            } else if constexpr (LIST) {
+                fvj = (loaded, ...);
             } else {
                 fvj = FV[j];
             }
@@ -316,7 +324,10 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
                                                           fold_lanes<LANES>(ud, mask);
                                                       });
         else if constexpr (LIST)
-            for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done, [] {});
+            for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done, [] {}, [&](int j) {
+                if constexpr (flat2<R, D>) return NoRecord{};
+                else return FV[j];
+            });
         else
             for_pairs<R, D, D == 3, false>(v, S, fr, P, i, P[i], body, cell_done);
     });

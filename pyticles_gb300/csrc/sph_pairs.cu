@@ -44,7 +44,7 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
     if (LANES == 1 && !active) return;
     with_masses<R, D, (LANES > 1)>(v, s, [&](auto same) {
         const PairMass<R, D, decltype(same)::value> mass(v, ii);
-        auto body = [&](int j, const T4 &pj, const R *d, R rsq, auto near) {
+        auto body = [&](int j, const T4 &pj, const R *d, R rsq, auto near, auto...) {
             const Dist<R> dd = plain_dist<R>(rsq);
             const R mj = mass(j, pj);
             R w, g;
@@ -68,7 +68,8 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
             // the entries of whole groups, less those that are no pairs
             const unsigned c = v.vl_cnt[i];
             cnt = (((c & 0xffffu) + 3) & ~3u) + (((c >> 16) + 3) & ~3u);
-            for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done, [&]() { --cnt; });
+            for_list<R, D, true>(v, S, fr, P, i, P[i], body, cell_done, [&]() { --cnt; },
+                                 [](int) { return NoRecord{}; });
         } else {
             for_pairs<R, D>(v, S, fr, P, i, P[i], body, cell_done);
         }
@@ -135,7 +136,7 @@ __device__ __forceinline__ void heat_one(const View &v, int i) {
     q[0].init(0);
     q[1].init(0);
     q[2].init(0);
-    auto body = [&](int j, const T4 &pj, const R *d, R rsq, auto) {
+    auto body = [&](int j, const T4 &pj, const R *d, R rsq, auto...) {
         R g = kernel_g<K, R, true>(ks, make_dist<R>(rsq));
         T4 fj = F[j];
         R dT = (fj.z - fi.z) + (fj.w - fi.w);
@@ -165,7 +166,9 @@ __device__ __forceinline__ void heat_one(const View &v, int i) {
                                                     if (D == 3) fold_lanes<LANES>(q[2], mask);
                                                 });
             if (!active || (threadIdx.x & (LANES - 1))) return;
-        } else if constexpr (LIST) for_list<R, D, false>(v, S, fr, P, i, P[i], body, cell_done, [] {});
+        } else if constexpr (LIST)
+            for_list<R, D, false>(v, S, fr, P, i, P[i], body, cell_done, [] {},
+                                  [](int) { return NoRecord{}; });
         else for_pairs<R, D, D == 3, false>(v, S, fr, P, i, P[i], body, cell_done);
     }
     R kap = sconst<R>(S).kappa;

@@ -297,10 +297,16 @@ __device__ __forceinline__ float vl_offset(unsigned k) {
 // particle itself three window cells away on every axis, which no pair within
 // the cutoff is, so that the walk tests no entry's place.  skip() is called for
 // every entry that is no pair, these among them.
-template <typename R, int D, bool FAR, typename T4, typename F, typename G, typename H>
+//
+// What the body needs of j beside its position record, load(j) fetches together
+// with that record, ahead of the pair test, and body gets it as its last
+// argument: most entries are pairs, so the loads are rarely wasted, and they do
+// not wait for the test.
+template <typename R, int D, bool FAR, typename T4, typename F, typename G, typename H,
+          typename L>
 __device__ __forceinline__ void for_list(const View &v, const SimDev &S,
                                          const PairFrame<R, D> &fr, const T4 *__restrict__ P,
-                                         int i, const T4 &pi, F body, G cell_done, H skip) {
+                                         int i, const T4 &pi, F body, G cell_done, H skip, L load) {
     static_assert(std::is_same<R, float>::value, "pair lists: mixed precision");
     constexpr int kBits = vl_index_bits(D);
     const unsigned cnt = v.vl_cnt[i];
@@ -313,6 +319,7 @@ __device__ __forceinline__ void for_list(const View &v, const SimDev &S,
         const float fx = vl_offset(t & 7u);
         const float fy = vl_offset(D == 3 ? (t >> 3) & 7u : t >> 3);
         const T4 pj = P[j];
+        const auto rec = load(j);
         R d[3];
         d[0] = __fmaf_rn(fx, fr.edge_lo[0], __fmaf_rn(fx, fr.edge[0], __fsub_rn(pj.x, pi.x)));
         d[1] = __fmaf_rn(fy, fr.edge_lo[1], __fmaf_rn(fy, fr.edge[1], __fsub_rn(pj.y, pi.y)));
@@ -328,7 +335,7 @@ __device__ __forceinline__ void for_list(const View &v, const SimDev &S,
             skip();
             return;
         }
-        body(j, pj, d, rsq, near);
+        body(j, pj, d, rsq, near, rec);
     };
     // the groups from pointer g, stepping `dir` rows each; slots in order
     // 0..3 (near) or 3..0 (far).  Measured on the 2D fluid: a lookahead of
@@ -361,6 +368,9 @@ __device__ __forceinline__ void for_list(const View &v, const SimDev &S,
         walk(E + (long long)((v.vl_cap >> 2) - 1) * st, -st, nf, std::false_type{},
              std::true_type{});
 }
+
+// load() of a list pass that needs the position records alone.
+struct NoRecord {};
 
 // Blocks of a pair-pass launch: one thread per particle, or with v.persist
 // only the blocks the device holds at once (SMs x resident blocks of this
