@@ -635,9 +635,15 @@ int alloc_cells(sph_engine *e, int64_t cells) {
     return SPH_OK;
 }
 
-// 2D mixed precision: velocities in the position records, the masses in what
-// are the velocity records otherwise (they do not change between stages).
+// 2D mixed precision: velocities in the position records; the buffers that hold
+// the velocity records otherwise have the masses (buffer 0 alone: they do not
+// change between stages) in their first half and the positions by themselves,
+// two floats a particle, in the second.
 bool flat2_layout(const sph_engine *e) { return e->dim == 2 && e->precision == SPH_MIXED; }
+// The velocity records of buffer b, in the flat layout its positions.
+void *vel_records(const sph_engine *e, int b) {
+    return flat2_layout(e) ? (char *)e->pk_vel[b] + 8 * e->cap_p : (char *)e->pk_vel[b];
+}
 
 View make_view(const sph_engine *e) {
     View v;
@@ -783,9 +789,9 @@ int vl_setup(sph_engine *e) {
 void stage_view(const sph_engine *e, View &v, int s) {
     int pin = s & 1, pout = (s + 1) & 1;
     v.pk_pos_in = e->pk_pos[pin];
-    v.pk_vel_in = e->pk_vel[pin];
+    v.pk_vel_in = vel_records(e, pin);
     v.pk_pos_out = e->pk_pos[pout];
-    v.pk_vel_out = e->pk_vel[pout];
+    v.pk_vel_out = vel_records(e, pout);
     for (int a = 0; a < 3; ++a) {
         v.xe_in[a] = s == 0 ? e->b_pos[a] : e->xe[(s - 1) & 1][a];
         v.xe_out[a] = e->xe[s & 1][a];
@@ -921,7 +927,7 @@ void enqueue_prepare(sph_engine *e, cudaStream_t st, bool gated = false, bool li
     View v = make_view(e);
     stage_view(e, v, 0);
     v.pk_pos_out = e->pk_pos[0];
-    v.pk_vel_out = e->pk_vel[0];
+    v.pk_vel_out = vel_records(e, 0);
     const int *gate = gated ? e->rebin_gate : nullptr;
     v.rebin_gate = gated ? e->rebin_gate : nullptr;
     if (gated)

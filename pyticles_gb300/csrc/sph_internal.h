@@ -146,7 +146,8 @@ struct View {
     double *org[3];         // B order: FP64 origin of the particle's cell-local frame
     // evaluation (stage s reads *_in, its force pass writes stage s+1's *_out)
     // packed positions and velocities, float4 / double4: {xl, yl, zl, m} and
-    // {vx, vy, vz, 0}; 2D mixed precision: {xl, yl, vx, vy}, the masses in pk_m
+    // {vx, vy, vz, 0}; 2D mixed precision: {xl, yl, vx, vy} and, as float2,
+    // {xl, yl}, the masses in pk_m
     void *pk_pos_in, *pk_vel_in;
     void *pk_pos_out, *pk_vel_out;
     void *pk_f, *pk_q;               // {p/rho^2, rho, T_hi, T_lo}, {q/rho^2, rho}

@@ -197,7 +197,10 @@ extern "C" int sph_derivatives_noalloc(const sph_params *p, int32_t precision, i
     w.steps = c.take<long long>(1);
     w.n_items = c.take<int>(1);
     w.mass_mixed = c.take<int>(1);
-    if (dim == 2 && precision == SPH_MIXED) w.pk_m = (float *)w.pk_vel_in;
+    if (dim == 2 && precision == SPH_MIXED) {   // the flat layout: masses, then positions
+        w.pk_m = (float *)w.pk_vel_in;
+        w.pk_vel_in = w.pk_vel_out = (char *)w.pk_vel_in + 8 * N;
+    }
     w.item_cell = w.rank;
     w.item_round = w.cell_of;
     w.items_max = (int)n;

@@ -24,7 +24,7 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
     bool active = i < v.np;
     const int ii = active ? i : v.np - 1;
     using T4 = typename V4<R>::T;
-    const T4 *__restrict__ P = (const T4 *)v.pk_pos_in;
+    const auto *__restrict__ P = positions<R, D>(v);
     const int s = v.b_sim[ii];
     const SimDev &S = ONE ? v.one : v.sims[s];
     if (S.cl_on || (!LIST && S.tile_on)) {   // cluster passes, cell tiles
@@ -44,7 +44,7 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
     if (LANES == 1 && !active) return;
     with_masses<R, D, (LANES > 1)>(v, s, [&](auto same) {
         const PairMass<R, D, decltype(same)::value> mass(v, ii);
-        auto body = [&](int j, const T4 &pj, const R *d, R rsq, auto near, auto...) {
+        auto body = [&](int j, const auto &pj, const R *d, R rsq, auto near, auto...) {
             const Dist<R> dd = plain_dist<R>(rsq);
             const R mj = mass(j, pj);
             R w, g;

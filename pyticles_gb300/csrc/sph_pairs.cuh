@@ -87,7 +87,8 @@ __device__ __forceinline__ bool pair_cell(const View &v, const SimDev &S,
     // rounding instead of the edge's rounding times the cell count
     R ox_ = (R)ox * fr.edge[0] - pi.x;
     R oy_ = (R)oy * fr.edge[1] - pi.y;
-    R oz_ = (D == 3) ? (R)oz * fr.edge[2] - pi.z : (R)0;
+    R oz_ = (R)0;
+    if constexpr (D == 3) oz_ = (R)oz * fr.edge[2] - pi.z;
     if constexpr (std::is_same<R, float>::value) {
         ox_ = __fmaf_rn((R)ox, fr.edge_lo[0], ox_);
         oy_ = __fmaf_rn((R)oy, fr.edge_lo[1], oy_);
@@ -109,7 +110,8 @@ __device__ __forceinline__ bool pair_cell(const View &v, const SimDev &S,
             R d[3];
             d[0] = pj.x + ox_;
             d[1] = pj.y + oy_;
-            d[2] = (D == 3) ? pj.z + oz_ : (R)0;
+            d[2] = (R)0;
+            if constexpr (D == 3) d[2] = pj.z + oz_;
             if constexpr (decltype(mi)::value) fr.min_image(d);
             R rsq = fma_(d[1], d[1], d[0] * d[0]);
             if (D == 3) rsq = fma_(d[2], d[2], rsq);
@@ -177,7 +179,7 @@ __device__ __forceinline__ void for_pairs(const View &v, const SimDev &S,
     for (int oz = -w2; oz <= w2; ++oz) {
         R dz = (R)0;
         int z = 0;
-        if (D == 3) {
+        if constexpr (D == 3) {
             dz = fmaxf_((R)oz * fr.edge[2] - pi.z, fr.ext[2]);
             z = c2 + oz;
             z += (z < 0) ? n2 : 0;
@@ -235,7 +237,8 @@ __device__ __forceinline__ void for_pairs_lanes(const View &v, const SimDev &S,
             const int oy = (D == 3 ? row % e1 : row) - w1, oz = D == 3 ? row / e1 - w2 : 0;
             const R dx = fmaxf_((R)ox * fr.edge[0] - pi.x, fr.ext[0]);
             const R dy = fmaxf_((R)oy * fr.edge[1] - pi.y, fr.ext[1]);
-            const R dz = D == 3 ? fmaxf_((R)oz * fr.edge[2] - pi.z, fr.ext[2]) : (R)0;
+            R dz = (R)0;
+            if constexpr (D == 3) dz = fmaxf_((R)oz * fr.edge[2] - pi.z, fr.ext[2]);
             const R dyz = fma_(dz, dz, dy * dy);
             const R dxyz = fma_(dx, dx, dyz);
             if (!(dyz > fr.thr_hi) && !(dxyz > fr.thr_hi)) {
@@ -325,7 +328,7 @@ __device__ __forceinline__ void for_list(const View &v, const SimDev &S,
         d[1] = __fmaf_rn(fy, fr.edge_lo[1], __fmaf_rn(fy, fr.edge[1], __fsub_rn(pj.y, pi.y)));
         d[2] = (R)0;
         R rsq = fma_(d[1], d[1], d[0] * d[0]);
-        if (D == 3) {
+        if constexpr (D == 3) {
             const float fz = vl_offset(t >> 6);
             d[2] = __fmaf_rn(fz, fr.edge_lo[2], __fmaf_rn(fz, fr.edge[2], __fsub_rn(pj.z, pi.z)));
             rsq = fma_(d[2], d[2], rsq);

@@ -31,8 +31,9 @@ __global__ void __launch_bounds__(256) k_vlist_build(const __grid_constant__ Vie
     const int s = v.b_sim[ii];
     const SimDev &S = v.one_sim ? v.one : v.sims[s];
     const SimConst<float> &c = S.cf;
-    const float4 *__restrict__ P = (const float4 *)v.pk_pos_in;
-    const float4 pi = P[ii];
+    const auto *__restrict__ P = positions<float, D>(v);
+    float4 pi = make_float4(P[ii].x, P[ii].y, 0.0f, 0.0f);
+    if constexpr (D == 3) pi = P[ii];
     int nn = 0, nf = 0;   // entries found
     int wn = 0, wf = 0;   // entries within the rows
     if (active) {
@@ -87,10 +88,10 @@ __global__ void __launch_bounds__(256) k_vlist_build(const __grid_constant__ Vie
                     const int tag = (int)(t << kBits);
                     for (int j = jb; j < je; ++j) {
                         if (j == i) continue;
-                        const float4 pj = P[j];
+                        const auto pj = P[j];
                         const float ddx = pj.x + ox_, ddy = pj.y + oy_;
                         float rsq = ddx * ddx + ddy * ddy;
-                        if (D == 3) {
+                        if constexpr (D == 3) {
                             const float ddz = pj.z + oz_;
                             rsq += ddz * ddz;
                         }
