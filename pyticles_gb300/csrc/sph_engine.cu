@@ -917,7 +917,10 @@ struct ProfScope {
     }
 };
 
-constexpr int kSortKernels = 7;  // bin, 3 scan, scatter, in-cell order, permute
+// Launches of the binning and the permutation, with the gated form's fill.
+int sort_kernels(const sph_engine *e) {
+    return binning_kernels(e->a_extent, e->ncells_total, rebin_on_demand(e)) + 1;
+}
 
 // Counting sort of A into B plus the packed first-evaluation copies.  Gated:
 // the kernels run only if the device gate is raised (binning on demand); the
@@ -930,15 +933,8 @@ void enqueue_prepare(sph_engine *e, cudaStream_t st, bool gated = false, bool li
     v.pk_vel_out = vel_records(e, 0);
     const int *gate = gated ? e->rebin_gate : nullptr;
     v.rebin_gate = gated ? e->rebin_gate : nullptr;
-    if (gated)
-        launch_fill_int(e->cell_count, 0, std::max(e->ncells_total, 1), st, gate);
-    else
-        cudaMemsetAsync(e->cell_count, 0, sizeof(int) * std::max(e->ncells_total, 1), st);
     cudaMemsetAsync(e->pair_count, 0, sizeof(unsigned long long) * e->cap_s, st);
-    launch_bin(v, e->a_extent, st);
-    launch_scan(e->cell_count, e->cell_start, e->ncells_total, e->scan_tmp, st, gate, e->n_items);
-    launch_scatter(v, e->a_extent, st);
-    launch_cellsort(v, e->ncells_total, st);
+    launch_binning(v, e->a_extent, e->ncells_total, e->scan_tmp, gate, st);
     launch_permute(v, e->precision, st);
     // a binning renumbers the slots: the pair lists are built again
     if (lists && e->vl.on && e->vl.ent && e->vl.cap > 0)
@@ -1197,21 +1193,21 @@ int64_t kernels_per_step(const sph_engine *e) {
         // cluster build; per evaluation density, [heat,] force and the stage
         // update; the later evaluations' repacking; the cell-window passes of
         // the other simulations
-        int64_t k = kSortKernels + cluster_build_kernels();
+        int64_t k = sort_kernels(e) + cluster_build_kernels();
         k += (int64_t)e->nstage * (3 + (e->group.heat_flux ? 1 : 0)) + (e->nstage - 1);
         if (e->n_cell_sims > 0)
             k += (int64_t)e->nstage * (2 + (e->group.heat_flux ? 1 : 0)) * forms;
         if (e->any_thermostat) k += 2;
-        if (rebin_on_demand(e)) k += 2;
+        if (rebin_on_demand(e)) ++k;   // the close
         return k;
     }
-    int64_t k = kSortKernels + (e->vl.on ? 1 : 0);   // + the pair lists' build
+    int64_t k = sort_kernels(e) + (e->vl.on ? 1 : 0);   // + the pair lists' build
     k += (int64_t)e->nstage * (2 + (e->group.heat_flux ? 1 : 0)) * (e->vl.on ? 1 : forms);
     if (e->any_thermostat) k += 2;
     // collisions: per find 5 kernels + 7 for the levels, one apply per
     // evaluation plus the extra first one, one integrator pass per stage
     if (e->group.collision != SPH_COLLIDE_OFF) k += (int64_t)e->nstage * 14 + 1;
-    if (rebin_on_demand(e)) k += 2;   // gated cell-count fill and close
+    if (rebin_on_demand(e)) ++k;   // the gated binning's close
     return k;
 }
 
@@ -2117,7 +2113,7 @@ int sph_profile_read(sph_engine *e, double ms[5], int64_t launches[5]) {
             continue;
         }
         ms[r.kind] += t;
-        launches[r.kind] += r.kind == SPH_PASS_SORT ? kSortKernels : (r.kind == SPH_PASS_TSUM ? 2 : 1);
+        launches[r.kind] += r.kind == SPH_PASS_SORT ? sort_kernels(e) : (r.kind == SPH_PASS_TSUM ? 2 : 1);
     }
     return SPH_OK;
 }

@@ -343,12 +343,15 @@ void launch_integrate(const View &v, int precision, int integrator, int stage, c
                       int cl_only = 0);
 
 // ---- launch wrappers (sph_sort.cu) ----
-void launch_bin(const View &v, int np_a, cudaStream_t s);
 // (clear: a counter set to 0 on the way, or null)
 void launch_scan(int *count, int *start, int n, int *block_tmp, cudaStream_t s,
                  const int *gate = nullptr, int *clear = nullptr);
-void launch_scatter(const View &v, int np_a, cudaStream_t s);
-void launch_cellsort(const View &v, int ncells, cudaStream_t s);
+// The counting sort of A's first np_a slots into ncells cells up to the canonical
+// order (v.order, v.cell_b, v.cell_start and the tile items), which
+// launch_permute applies; gated by *gate if given.  binning_kernels: its launches.
+void launch_binning(const View &v, int np_a, int ncells, int *scan_tmp, const int *gate,
+                    cudaStream_t s);
+int binning_kernels(int np_a, int ncells, bool gated);
 void launch_permute(const View &v, int precision, cudaStream_t s);
 // A simulation's state just set in A (identity order from a_off) into its B
 // slots [b0, b0 + n) of the current binning; raises *far if it needs a new

@@ -221,7 +221,6 @@ extern "C" int sph_derivatives_noalloc(const sph_params *p, int32_t precision, i
     NA_CK(cudaMemsetAsync(w.err, 0, sizeof(int), st));
     NA_CK(cudaMemsetAsync(w.err_any, 0, sizeof(int), st));
     NA_CK(cudaMemsetAsync(w.pair_count, 0, sizeof(unsigned long long), st));
-    NA_CK(cudaMemsetAsync(w.cell_count, 0, sizeof(int) * ncells, st));
     NA_CK(cudaMemsetAsync(w.pk_q, 0, N * v4, st));
     launch_load_aos(w.a_pos, r, (int)n, dim, st);
     launch_load_aos(w.a_vel, v, (int)n, dim, st);
@@ -230,10 +229,7 @@ extern "C" int sph_derivatives_noalloc(const sph_params *p, int32_t precision, i
     launch_iota_sim(w.a_id, w.a_sim, 0, (int)n, w.a_m, w.mass_mixed, st);
 
     // the engine's passes: counting sort, density, heat, force (no state update)
-    launch_bin(w, (int)n, st);
-    launch_scan(w.cell_count, w.cell_start, ncells, scan_tmp, st, nullptr, w.n_items);
-    launch_scatter(w, (int)n, st);
-    launch_cellsort(w, ncells, st);
+    launch_binning(w, (int)n, ncells, scan_tmp, nullptr, st);
     launch_permute(w, precision, st);
     launch_density(w, precision, p->kernel, 0, 128, st);
     if (p->heat_flux) launch_heat(w, precision, p->kernel, 128, st);
