@@ -195,6 +195,19 @@ __device__ __forceinline__ void integrate_stage(const View &v, const SimDev &S, 
     }
 }
 
+// Epilogue of the force passes: the rates of particle i and, with mode, its
+// integrator stage.
+template <typename R, int D>
+__device__ __forceinline__ void force_finish(const View &v, const SimDev &S, int i, int s, int stage,
+                                             int mode, int integ, const R *vdr, R udr) {
+    for (int a = 0; a < D; ++a) ((R *)v.vdot[a])[i] = vdr[a];
+    ((R *)v.udot)[i] = udr;
+    if (!isfinite(vdr[0]) || !isfinite(udr)) set_err(v.err, v.err_any, s, SPH_ENAN);
+    if (mode == 0) return;
+
+    integrate_stage<R, D>(v, S, i, s, stage, integ, vdr, udr);
+}
+
 // VH: bit 0 viscosity, bit 1 heat flux (compile-time, so a workload without
 // them carries neither their registers nor their branches).  ONE: a single
 // simulation, whose constants come from the kernel parameters.
@@ -331,15 +344,25 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
         else
             for_pairs<R, D, D == 3, false>(v, S, fr, P, i, P[i], body, cell_done);
     });
-    if (LANES > 1 && (!active || (threadIdx.x & (LANES - 1)))) return;
     R vdr[3] = {ax[0].get(), ax[1].get(), ax[2].get()};
     R udr = (R)0.5 * ud.get();
-    for (int a = 0; a < D; ++a) ((R *)v.vdot[a])[i] = vdr[a];
-    ((R *)v.udot)[i] = udr;
-    if (!isfinite(vdr[0]) || !isfinite(udr)) set_err(v.err, v.err_any, s, SPH_ENAN);
-    if (mode == 0) return;
-
-    integrate_stage<R, D>(v, S, i, s, stage, integ, vdr, udr);
+    if constexpr (LANES > 1) {   // the epilogue by consecutive threads (lanes_block)
+        constexpr int N = lanes_block<LANES> / LANES;   // particles of the block
+        __shared__ float4 rates[N];
+        __shared__ int live[N];
+        if ((threadIdx.x & (LANES - 1)) == 0) {
+            rates[threadIdx.x / LANES] = make_float4(vdr[0], vdr[1], vdr[2], udr);
+            live[threadIdx.x / LANES] = active;
+        }
+        __syncthreads();
+        const int t = threadIdx.x, p = blockIdx.x * N + t;
+        if (t >= N || !live[t]) return;
+        const R vd[3] = {rates[t].x, rates[t].y, rates[t].z};
+        const int sp = v.b_sim[p];
+        force_finish<R, D>(v, v.sims[sp], p, sp, stage, mode, integ, vd, rates[t].w);
+    } else {
+        force_finish<R, D>(v, S, i, s, stage, mode, integ, vdr, udr);
+    }
 }
 
 // One thread per particle; PERSIST: the resident blocks of pass_grid walk
@@ -410,9 +433,9 @@ void force_launch(const View &v, int stage, int mode, int integ, int block, cuda
         k_force_vl<D, K, VH, ONE><<<grid, block, 0, s>>>(v, stage, mode, integ);
     } else if constexpr (FORM == kForceLanes) {
         if (walk_lanes(v) == 32)
-            k_force_lanes<D, K, VH, 32><<<lanes_grid(v, 32), 128, 0, s>>>(v, stage, mode, integ);
+            k_force_lanes<D, K, VH, 32><<<lanes_grid<32>(v), lanes_block<32>, 0, s>>>(v, stage, mode, integ);
         else
-            k_force_lanes<D, K, VH, 8><<<lanes_grid(v, 8), 128, 0, s>>>(v, stage, mode, integ);
+            k_force_lanes<D, K, VH, 8><<<lanes_grid<8>(v), lanes_block<8>, 0, s>>>(v, stage, mode, integ);
     } else if (std::is_same<R, float>::value && v.persist) {
         auto *fn = k_force<R, D, K, VH, ONE, std::is_same<R, float>::value>;
         fn<<<pass_grid(v, fn, block), block, 0, s>>>(v, stage, mode, integ);

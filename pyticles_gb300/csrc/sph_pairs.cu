@@ -77,9 +77,24 @@ __device__ __forceinline__ void density_one(const View &v, int stage, int i) {
     if constexpr (LANES > 1) {
 #pragma unroll
         for (int o = LANES / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        if (!active || (threadIdx.x & (LANES - 1))) return;
+        // the epilogue by consecutive threads (lanes_block)
+        constexpr int N = lanes_block<LANES> / LANES;   // particles of the block
+        __shared__ double sum_s[N], sum_l[N];
+        __shared__ unsigned pairs[N];
+        if ((threadIdx.x & (LANES - 1)) == 0) {
+            const int t = threadIdx.x / LANES;
+            sum_s[t] = rs.get64();
+            sum_l[t] = rl.get64();
+            pairs[t] = active ? cnt : ~0u;
+        }
+        __syncthreads();
+        const int t = threadIdx.x, p = blockIdx.x * N + t;
+        if (t >= N || pairs[t] == ~0u) return;
+        const int sp = v.b_sim[p];
+        density_finish<R, D>(v, v.sims[sp], p, sp, stage, sum_s[t], sum_l[t], pairs[t]);
+    } else {
+        density_finish<R, D>(v, S, i, s, stage, rs.get64(), rl.get64(), cnt);
     }
-    density_finish<R, D>(v, S, i, s, stage, rs.get64(), rl.get64(), cnt);
 }
 
 // One thread per particle; PERSIST: the resident blocks of pass_grid walk
@@ -223,11 +238,11 @@ void density_launch(const View &v, int stage, int block, cudaStream_t s) {
         }
         const int lanes = walk_lanes(v);
         if (lanes == 32) {
-            k_density_lanes<D, K, 32><<<lanes_grid(v, 32), 128, 0, s>>>(v, stage);
+            k_density_lanes<D, K, 32><<<lanes_grid<32>(v), lanes_block<32>, 0, s>>>(v, stage);
             return;
         }
         if (lanes == 8) {
-            k_density_lanes<D, K, 8><<<lanes_grid(v, 8), 128, 0, s>>>(v, stage);
+            k_density_lanes<D, K, 8><<<lanes_grid<8>(v), lanes_block<8>, 0, s>>>(v, stage);
             return;
         }
     }
@@ -248,11 +263,11 @@ void heat_launch(const View &v, int block, cudaStream_t s) {
         }
         const int lanes = walk_lanes(v);
         if (lanes == 32) {
-            k_heat_lanes<D, K, 32><<<lanes_grid(v, 32), 128, 0, s>>>(v);
+            k_heat_lanes<D, K, 32><<<lanes_grid<32>(v), lanes_block<32>, 0, s>>>(v);
             return;
         }
         if (lanes == 8) {
-            k_heat_lanes<D, K, 8><<<lanes_grid(v, 8), 128, 0, s>>>(v);
+            k_heat_lanes<D, K, 8><<<lanes_grid<8>(v), lanes_block<8>, 0, s>>>(v);
             return;
         }
     }

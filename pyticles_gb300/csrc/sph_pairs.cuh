@@ -394,8 +394,16 @@ template <typename F> inline int pass_grid(const View &v, F *kernel, int block) 
 // 816; 3D with heat flux 2,197 particles 2122 / 615 / 274, 8,000 2124 / 608 / 675,
 // 32,768 2354 / 1923 / 2505, 64,000 2377 / 3041 / 4484.
 inline int walk_lanes(const View &v) { return v.np <= 4096 ? 32 : (v.np <= 40960 ? 8 : 1); }
-inline int lanes_grid(const View &v, int lanes) {   // blocks of 128 threads
-    return (int)(((long long)v.np * lanes + 127) / 128);
+// Threads per block, and blocks, of the passes with LANES lanes per particle.  Their
+// epilogues (FP64, an instruction of which costs the pipe the same for one lane of a
+// warp as for all) are done by the block's first threads, one per particle, from
+// shared memory.  Density + force of a step, us, epilogue by each particle's first
+// lane / so in blocks of 128 / of 256: 2D 32 lanes 4k particles 102.4 / 85.5 / 88.1,
+// 1k 70.2 / 68.4 / 68.6; 8 lanes 9k 106.0 / 105.4 / 102.6, 22k 179.8 / 173.1 / 171.1; 3D
+// with heat 32 lanes 1.7k 241 / 243 / 248, 8 lanes 16k 1010 / 1007 / 990.
+template <int LANES> constexpr int lanes_block = LANES == 32 ? 128 : 256;
+template <int LANES> inline int lanes_grid(const View &v) {
+    return (int)(((long long)v.np * LANES + lanes_block<LANES> - 1) / lanes_block<LANES>);
 }
 
 // Warp-aggregated per-simulation counter update.
