@@ -359,17 +359,25 @@ double fast_margin(const sph_engine *e, const Sim &S, const SimDev &d) {
     return ulp * (16.0 + 4.0 * 2.0 * std::sqrt((double)e->dim) * most / std::sqrt(d.thr));
 }
 
-// Cell tiles serve simulations whose cells hold at least two particles on
-// average (a block fills its tile once per cell, and a nearly empty cell does
-// not repay it).  The rules are of the simulation alone, so its bits are too.
-bool tile_scheme(int precision, int64_t n, int ncells) {
-    return precision == SPH_FP64 && n >= 2 * (int64_t)ncells;
+// Cell tiles serve small FP64 simulations, and larger ones whose cells hold two
+// particles (2D) or one (3D) on average: a block fills its tile once per cell, and a
+// nearly empty cell does not repay it, while a small launch is bound by latency, which
+// the tiles spread over more lanes.  Step of a simulation, us, walk / tiles, at
+// particles per cell: 2D 160,000 particles 5795 / 3781 at 2.25, 4476 / 4855 at 1.56,
+// 1045 / 6037 at 0.25; 16,384 848 / 435, 688 / 560, 240 / 675; 1,024 825 / 70,
+// 671 / 90, 229 / 76; 3D with heat 32,768 6735 / 3714 at 1.37, 4156 / 4443 at 0.70,
+// 2506 / 4237 at 0.30; 2,197 4242 / 370, 2894 / 379, 1881 / 372.  The rules are of the
+// simulation alone, so its bits are too.
+constexpr int64_t kTileSmall = 3072;
+bool tile_scheme(int precision, int dim, int64_t n, int ncells) {
+    if (precision != SPH_FP64) return false;
+    return n <= kTileSmall || n >= (dim == 2 ? 2 : 1) * (int64_t)ncells;
 }
 // Lanes per particle (log2) of the cell tiles: 32 for a small simulation, which
 // spreads it over more warps, eight otherwise.  Density + force of a step, us,
 // 32 / 16 / 8 lanes: 2D 1,024 particles 94 / 107 / 112, 4,096 230 / 214 / 180;
 // 3D 2,197 particles 571 / 711 / 920, 8,000 1934 / 1691 / 1704.
-int tile_lanes(int64_t n) { return n <= 3072 ? 5 : 3; }
+int tile_lanes(int64_t n) { return n <= kTileSmall ? 5 : 3; }
 // Most work items of a simulation.
 int64_t tile_items(int64_t n, int ncells) {
     const int per = kTileRounds * (32 >> tile_lanes(n));
@@ -395,7 +403,7 @@ SimDev make_simdev(const sph_engine *e, const Sim &S) {
             (a < e->dim && S.win[a] > 0) ? 0.5 * S.edge[a] + 0.5 * d.slack_half[a] : 1e300;
         if (a < e->dim && S.nc[a] == 1) d.small_mask |= (1 << a);
     }
-    d.tile_on = tile_scheme(e->precision, S.n, S.ncells) ? 1 : 0;
+    d.tile_on = tile_scheme(e->precision, e->dim, S.n, S.ncells) ? 1 : 0;
     d.tile_lg = tile_lanes(S.n);
     d.vl_gate2 = S.vl_skin > 0.0 ? 0.0625 * S.vl_skin * S.vl_skin : 1e300;
     d.vl_eskin2 = S.vl_skin > 0.0 ? 0.25 * S.vl_skin * S.vl_skin : 1e300;
