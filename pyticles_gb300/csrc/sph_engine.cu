@@ -1696,6 +1696,9 @@ int sph_sim_set_state(sph_engine *e, int32_t id, const double *r, const double *
         CK(cudaMemsetAsync(e->restage_far, 0, sizeof(int), st));
         View vw = make_view(e);
         stage_view(e, vw, 0);
+        // into the records that the next step's first evaluation reads
+        vw.pk_pos_out = vw.pk_pos_in;
+        vw.pk_vel_out = vw.pk_vel_in;
         launch_restage(vw, e->precision, S.a_off, S.part_off, (int)S.n, e->restage_far, st);
         CK(cudaMemcpyAsync(&far, e->restage_far, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
