@@ -226,6 +226,10 @@ static void launch_cellsort(const View &v, int ncells, cudaStream_t s) {
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallParticles = 2048, kSmallCells = 8192;
 constexpr int kSmallPer = kSmallParticles / kSmallThreads;
+// Shared memory of a block without an opt-in is 48 KB, the static arrays (144
+// bytes, block_excl_scan) among them: 1 KB is left for those.
+constexpr int kSmallBytes = 47 * 1024;
+inline int small_bytes(int np_a, int ncells) { return (ncells + 2 * np_a) * (int)sizeof(int); }
 
 __global__ void __launch_bounds__(kSmallThreads) k_bin_small(View v, int np_a, int ncells) {
     if (v.rebin_gate && *v.rebin_gate == 0) return;
@@ -281,7 +285,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_bin_small(View v, int np_a, i
 }
 
 bool small_binning(int np_a, int ncells) {
-    return np_a <= kSmallParticles && ncells <= kSmallCells;
+    return np_a <= kSmallParticles && ncells <= kSmallCells &&
+           small_bytes(np_a, ncells) <= kSmallBytes;
 }
 
 int binning_kernels(int np_a, int ncells, bool gated) {
@@ -291,12 +296,7 @@ int binning_kernels(int np_a, int ncells, bool gated) {
 void launch_binning(const View &v, int np_a, int ncells, int *scan_tmp, const int *gate,
                     cudaStream_t s) {
     if (np_a > 0 && ncells > 0 && small_binning(np_a, ncells)) {
-        const int bytes = (ncells + 2 * np_a) * (int)sizeof(int);
-        constexpr int kMost = (kSmallCells + 2 * kSmallParticles) * (int)sizeof(int);
-        if (bytes > 48 * 1024)
-            cudaFuncSetAttribute(k_bin_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kMost);
-        k_bin_small<<<1, kSmallThreads, bytes, s>>>(v, np_a, ncells);
+        k_bin_small<<<1, kSmallThreads, small_bytes(np_a, ncells), s>>>(v, np_a, ncells);
         return;
     }
     if (gate) launch_fill_int(v.cell_count, 0, ncells > 1 ? ncells : 1, s, gate);
