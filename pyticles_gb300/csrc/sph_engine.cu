@@ -368,10 +368,17 @@ double fast_margin(const sph_engine *e, const Sim &S, const SimDev &d) {
 // 671 / 90, 229 / 76; 3D with heat 32,768 6735 / 3714 at 1.37, 4156 / 4443 at 0.70,
 // 2506 / 4237 at 0.30; 2,197 4242 / 370, 2894 / 379, 1881 / 372.  The rules are of the
 // simulation alone, so its bits are too.
+// The tiles test their candidates in FP32, so the squares of the simulation's lengths
+// must lie well inside its range; the window walk is FP64 throughout and takes the rest.
 constexpr int64_t kTileSmall = 3072;
-bool tile_scheme(int precision, int dim, int64_t n, int ncells) {
-    if (precision != SPH_FP64) return false;
-    return n <= kTileSmall || n >= (dim == 2 ? 2 : 1) * (int64_t)ncells;
+bool tile_scheme(const sph_engine *e, const Sim &S) {
+    if (e->precision != SPH_FP64) return false;
+    const sph_params &p = S.prm;
+    const double thr = p.cutoff * p.cutoff + p.tolerance * p.tolerance;
+    if (!(thr >= 1e-24 && thr <= 1e34)) return false;
+    for (int a = 0; a < e->dim; ++a)
+        if (p.box[a] > 1e17) return false;
+    return S.n <= kTileSmall || S.n >= (e->dim == 2 ? 2 : 1) * (int64_t)S.ncells;
 }
 // Lanes per particle (log2) of the cell tiles: 32 for a small simulation, which
 // spreads it over more warps, eight otherwise.  Density + force of a step, us,
@@ -403,7 +410,7 @@ SimDev make_simdev(const sph_engine *e, const Sim &S) {
             (a < e->dim && S.win[a] > 0) ? 0.5 * S.edge[a] + 0.5 * d.slack_half[a] : 1e300;
         if (a < e->dim && S.nc[a] == 1) d.small_mask |= (1 << a);
     }
-    d.tile_on = tile_scheme(e->precision, e->dim, S.n, S.ncells) ? 1 : 0;
+    d.tile_on = tile_scheme(e, S) ? 1 : 0;
     d.tile_lg = tile_lanes(S.n);
     d.vl_gate2 = S.vl_skin > 0.0 ? 0.0625 * S.vl_skin * S.vl_skin : 1e300;
     d.vl_eskin2 = S.vl_skin > 0.0 ? 0.25 * S.vl_skin * S.vl_skin : 1e300;

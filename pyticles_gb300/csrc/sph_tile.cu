@@ -141,10 +141,6 @@ template <int D, typename Rec> struct TileMem {
         }
         mass[k] = m;
     }
-    __device__ __forceinline__ void pad(int k) {   // fails every test
-#pragma unroll
-        for (int a = 0; a < D; ++a) t[a][k] = 1e18f;
-    }
 };
 // Each warp's queues of accepted candidates, one per particle of the round:
 // near pairs from the front, far ones from the back.
@@ -549,9 +545,6 @@ template <int D, typename Pass> struct Window {
             }
             T = T1;
         }
-        // candidates past the end fail every test
-        const int end = min(kTileCap, (T + 63) & ~63);
-        for (int k = T + (int)threadIdx.x; k < end; k += kTileThreads) mem.pad(k);
         __syncthreads();
     }
 };
@@ -595,6 +588,12 @@ __device__ __forceinline__ void tile_round(const View &v, const SimDev &S, Mem &
                 tile_test<D, false>(mem, k0 + l, G, steps, sn, pt, S.cf, thr, thr_s, 0, in, near);
             if (!live) in = 0u;
             const int top = k0 + l + (2 * steps - 1) * G;
+            // the test reads whole steps: slots past the tile's end hold no candidate
+            // (whatever an earlier tile left there, which must name no particle)
+            if (top >= win.T) {
+                const int past = (top - win.T) >> lg;
+                in &= past < 31 ? 0xfffffffeu << past : 0u;
+            }
             // a particle is not its own neighbour
             if (i >= win.s_first && i < win.s_last) {
                 const int up = top - (i - win.s_base), q = up >> lg;
