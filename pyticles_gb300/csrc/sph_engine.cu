@@ -288,6 +288,41 @@ void make_grid(Sim &S, int dim, double ratio, double list_skin = 0.0) {
     }
 }
 
+// Bound on the sum of an FP32 separation's roundings, over the axes: a position's
+// local coordinate has at most h (half its cell and the allowed drift), a window
+// cell's frame lies at most win edge + h away, and a separation takes at most four
+// roundings of such magnitudes per axis.
+double fast_reach(const sph_engine *e, const Sim &S, const SimDev &d) {
+    double most = 0.0;
+    for (int a = 0; a < e->dim; ++a) {
+        const double h = S.win[a] > 0 ? d.box_half[a] : 0.5 * d.L[a];
+        const double reach = S.win[a] > 0 ? S.win[a] * S.edge[a] : d.L[a];
+        most = std::max(most, 4.0 * (reach + 3.0 * h));
+    }
+    return std::sqrt((double)e->dim) * most;
+}
+
+// Relative half width of the guard band around the cutoff in FP32: four times a
+// bound on what rounding can move an FP32 squared distance at the cutoff; 16 more
+// units cover the squares and sums.  5e-6 for the 2D fluid (measured error below 1e-6).
+// Every pair inside the band pays the FP64 test with a warp to itself: a band of
+// 2^-12 kept the FP64 pipe of the 3D list density pass 43% busy.
+constexpr double kUlp32 = 1.0 / 16777216.0;
+double fast_margin(const sph_engine *e, const Sim &S, const SimDev &d) {
+    return kUlp32 * (16.0 + 4.0 * 2.0 * fast_reach(e, S, d) / std::sqrt(d.thr));
+}
+
+// The square of a compact short kernel's support, grown so that no pair within the
+// support is filed beyond it: by 2^-10, which covers the FP32 kernels' own rounding,
+// or by four times the bound on an FP32 squared distance's error at the support,
+// which is more in cells or boxes some thousand supports wide (drift room of fast
+// particles, single-cell axes).
+double short_support2(const sph_engine *e, const Sim &S, const SimDev &d, double supp) {
+    const double move = 4.0 * kUlp32 * fast_reach(e, S, d);
+    return supp * supp +
+           std::max(supp * supp / 1024.0, 16.0 * kUlp32 * supp * supp + 2.0 * supp * move + move * move);
+}
+
 template <typename R>
 void fill_const(SimConst<R> &c, const sph_engine *e, const Sim &S, const SimDev &d,
                 double margin) {
@@ -296,10 +331,10 @@ void fill_const(SimConst<R> &c, const sph_engine *e, const Sim &S, const SimDev 
     c.thr_hi = (R)(d.thr * (1.0 + margin));
     // compact short kernels vanish beyond h (Lucy, Debrun) or 2h (cubic); the
     // margin keeps every pair the FP32 kernel could still see as q < 1
-    double supp = p.kernel == SPH_KERNEL_CUBIC ? 2.0 * p.h_short : p.h_short;
+    const double supp = p.kernel == SPH_KERNEL_CUBIC ? 2.0 * p.h_short : p.h_short;
+    const double supp2 = short_support2(e, S, d, supp);
     c.thr_s = c.thr_hi;
-    if (p.kernel != SPH_KERNEL_GAUSSIAN && supp * supp * (1.0 + 1.0 / 1024.0) < d.thr)
-        c.thr_s = (R)(supp * supp * (1.0 + 1.0 / 1024.0));
+    if (p.kernel != SPH_KERNEL_GAUSSIAN && supp2 < d.thr) c.thr_s = (R)supp2;
     for (int a = 0; a < 3; ++a) {
         c.edge[a] = (R)S.edge[a];
         c.edge_lo[a] = (R)(S.edge[a] - (double)c.edge[a]);
@@ -316,8 +351,8 @@ void fill_const(SimConst<R> &c, const sph_engine *e, const Sim &S, const SimDev 
         const double rc = std::sqrt(d.thr), sk = S.vl_skin;
         c.vl_thr = (R)((rc + sk) * (rc + sk) * (1.0 + 1.0 / 1024.0));
         double near = (rc + sk) * (rc + sk);
-        if (p.kernel != SPH_KERNEL_GAUSSIAN && supp * supp * (1.0 + 1.0 / 1024.0) < d.thr) {
-            const double sq = supp * std::sqrt(1.0 + 1.0 / 1024.0);
+        if (p.kernel != SPH_KERNEL_GAUSSIAN && supp2 < d.thr) {
+            const double sq = std::sqrt(supp2);
             near = std::min(near, (sq + sk) * (sq + sk));
         }
         c.vl_near = (R)(near * (1.0 + 1.0 / 1024.0));
@@ -338,25 +373,6 @@ void fill_const(SimConst<R> &c, const sph_engine *e, const Sim &S, const SimDev 
     c.g0_pl = (R)(g0l * (-2.0 * p.adash));
     c.g0_h2_pl = (R)(g0l / (p.h_long * p.h_long) * (-2.0 * p.adash));
     c.kappa = (R)p.thermalk;
-}
-
-// Relative half width of the guard band around the cutoff in FP32: four times a
-// bound on what rounding can move an FP32 squared distance at the cutoff.  A
-// position's local coordinate has at most h (half its cell and the allowed
-// drift), a window cell's frame lies at most win edge + h away, and a separation
-// takes at most four roundings of such magnitudes per axis; 16 more units cover
-// the squares and sums.  5e-6 for the 2D fluid (measured error below 1e-6).
-// Every pair inside the band pays the FP64 test with a warp to itself: a band of
-// 2^-12 kept the FP64 pipe of the 3D list density pass 43% busy.
-double fast_margin(const sph_engine *e, const Sim &S, const SimDev &d) {
-    double most = 0.0;
-    for (int a = 0; a < e->dim; ++a) {
-        const double h = S.win[a] > 0 ? d.box_half[a] : 0.5 * d.L[a];
-        const double reach = S.win[a] > 0 ? S.win[a] * S.edge[a] : d.L[a];
-        most = std::max(most, 4.0 * (reach + 3.0 * h));
-    }
-    const double ulp = 1.0 / 16777216.0;
-    return ulp * (16.0 + 4.0 * 2.0 * std::sqrt((double)e->dim) * most / std::sqrt(d.thr));
 }
 
 // Cell tiles serve small FP64 simulations, and larger ones whose cells hold two
