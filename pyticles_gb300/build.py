@@ -18,7 +18,7 @@ SOURCES = ["sph_engine.cu", "sph_sort.cu", "sph_pairs.cu", "sph_force_f32.cu",
            "sph_force_f64.cu", "sph_noalloc.cu", "sph_splat.cu", "sph_collide.cu",
            "sph_cluster.cu", "sph_kfunc.cu", "sph_vlist.cu", "sph_tile.cu",
            "sph_force_walk2.cu", "sph_force_walk3.cu", "sph_force_lanes2.cu", "sph_force_lanes3.cu",
-           "sph_force_list.cu"]
+           "sph_force_list.cu", "sph_force_lanes64_2.cu", "sph_force_lanes64_3.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
          "--expt-relaxed-constexpr"]

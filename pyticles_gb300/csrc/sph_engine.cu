@@ -375,18 +375,18 @@ void fill_const(SimConst<R> &c, const sph_engine *e, const Sim &S, const SimDev 
     c.kappa = (R)p.thermalk;
 }
 
-// Cell tiles serve small FP64 simulations, and larger ones whose cells hold two
-// particles (2D) or one (3D) on average: a block fills its tile once per cell, and a
-// nearly empty cell does not repay it, while a small launch is bound by latency, which
-// the tiles spread over more lanes.  Step of a simulation, us, walk / tiles, at
-// particles per cell: 2D 160,000 particles 5795 / 3781 at 2.25, 4476 / 4855 at 1.56,
-// 1045 / 6037 at 0.25; 16,384 848 / 435, 688 / 560, 240 / 675; 1,024 825 / 70,
-// 671 / 90, 229 / 76; 3D with heat 32,768 6735 / 3714 at 1.37, 4156 / 4443 at 0.70,
-// 2506 / 4237 at 0.30; 2,197 4242 / 370, 2894 / 379, 1881 / 372.  The rules are of the
-// simulation alone, so its bits are too.
+// Cell tiles serve the FP64 simulations whose cells hold two particles (2D) or one (3D)
+// on average: a block fills its tile once per cell, and a nearly empty cell does not
+// repay it.  Step, us, window walk / tiles, at particles per cell: 2D 160,000 particles
+// 5795 / 3781 at 2.25, 4476 / 4855 at 1.56, 1045 / 6037 at 0.25; 150 simulations of 1,024
+// 5309 / 3990 at 2.56, 3970 / 5129 at 1.56, 1048 / 5929 at 0.25; 3D with heat 32,768 6735 /
+// 3714 at 1.37, 4156 / 4443 at 0.70, 2506 / 4237 at 0.30; 64 simulations of 2,197 14570 /
+// 13429 at 1.33, 6702 / 16996 at 0.61.  A small sparse simulation by itself would gain by
+// tiles (2D 1,024 at 1.56 130 / 87, 2,704 at 0.25 121 / 153; 3D 2,197 at 0.61 559 / 342,
+// the walk by several lanes per particle), but in a batch of them tiles lose by up to 5.7
+// times, and the rule is of the simulation alone, so that its bits are too.
 // The tiles test their candidates in FP32, so the squares of the simulation's lengths
 // must lie well inside its range; the window walk is FP64 throughout and takes the rest.
-constexpr int64_t kTileSmall = 3072;
 bool tile_scheme(const sph_engine *e, const Sim &S) {
     if (e->precision != SPH_FP64) return false;
     const sph_params &p = S.prm;
@@ -394,12 +394,13 @@ bool tile_scheme(const sph_engine *e, const Sim &S) {
     if (!(thr >= 1e-24 && thr <= 1e34)) return false;
     for (int a = 0; a < e->dim; ++a)
         if (p.box[a] > 1e17) return false;
-    return S.n <= kTileSmall || S.n >= (e->dim == 2 ? 2 : 1) * (int64_t)S.ncells;
+    return S.n >= (e->dim == 2 ? 2 : 1) * (int64_t)S.ncells;
 }
 // Lanes per particle (log2) of the cell tiles: 32 for a small simulation, which
 // spreads it over more warps, eight otherwise.  Density + force of a step, us,
 // 32 / 16 / 8 lanes: 2D 1,024 particles 94 / 107 / 112, 4,096 230 / 214 / 180;
 // 3D 2,197 particles 571 / 711 / 920, 8,000 1934 / 1691 / 1704.
+constexpr int64_t kTileSmall = 3072;
 int tile_lanes(int64_t n) { return n <= kTileSmall ? 5 : 3; }
 // Most work items of a simulation.
 int64_t tile_items(int64_t n, int ncells) {

@@ -348,10 +348,10 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
     R udr = (R)0.5 * ud.get();
     if constexpr (LANES > 1) {   // the epilogue by consecutive threads (lanes_block)
         constexpr int N = lanes_block<LANES> / LANES;   // particles of the block
-        __shared__ float4 rates[N];
+        __shared__ T4 rates[N];
         __shared__ int live[N];
         if ((threadIdx.x & (LANES - 1)) == 0) {
-            rates[threadIdx.x / LANES] = make_float4(vdr[0], vdr[1], vdr[2], udr);
+            rates[threadIdx.x / LANES] = make_v4<R>(vdr[0], vdr[1], vdr[2], udr);
             live[threadIdx.x / LANES] = active;
         }
         __syncthreads();
@@ -398,10 +398,10 @@ __global__ void __launch_bounds__(256, ONE ? (D == 2 ? SPH_VL_FORCE_BLOCKS : SPH
 }
 
 // The cell windows of a small launch, LANES lanes per particle.
-template <int D, int K, int VH, int LANES>
+template <typename R, int D, int K, int VH, int LANES>
 __global__ void __launch_bounds__(256)
     k_force_lanes(const __grid_constant__ View v, int stage, int mode, int integ) {
-    force_one<float, D, K, VH, false, false, LANES>(
+    force_one<R, D, K, VH, false, false, LANES>(
         v, stage, mode, integ, (blockIdx.x * blockDim.x + threadIdx.x) / LANES);
 }
 
@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(256) k_integrate(View v, int stage, int integ,
 
 // The forms of the force pass, each instantiated in a translation unit of its
 // own (sph_force_*.cu) per dimension.  The persistent form is for the
-// mixed-precision pass only (see density_launch); FP64 walks serve the
+// mixed-precision pass only (see density_launch); FP64 walks (and lanes) serve the
 // simulations that are too sparse for cell tiles.
 enum ForceForm { kForceWalk, kForceList, kForceLanes };
 
@@ -432,10 +432,10 @@ void force_launch(const View &v, int stage, int mode, int integ, int block, cuda
     if constexpr (FORM == kForceList) {
         k_force_vl<D, K, VH, ONE><<<grid, block, 0, s>>>(v, stage, mode, integ);
     } else if constexpr (FORM == kForceLanes) {
-        if (walk_lanes(v) == 32)
-            k_force_lanes<D, K, VH, 32><<<lanes_grid<32>(v), lanes_block<32>, 0, s>>>(v, stage, mode, integ);
+        if (walk_lanes<R>(v) == 32)
+            k_force_lanes<R, D, K, VH, 32><<<lanes_grid<32>(v), lanes_block<32>, 0, s>>>(v, stage, mode, integ);
         else
-            k_force_lanes<D, K, VH, 8><<<lanes_grid<8>(v), lanes_block<8>, 0, s>>>(v, stage, mode, integ);
+            k_force_lanes<R, D, K, VH, 8><<<lanes_grid<8>(v), lanes_block<8>, 0, s>>>(v, stage, mode, integ);
     } else if (std::is_same<R, float>::value && v.persist) {
         auto *fn = k_force<R, D, K, VH, ONE, std::is_same<R, float>::value>;
         fn<<<pass_grid(v, fn, block), block, 0, s>>>(v, stage, mode, integ);

@@ -13,6 +13,8 @@ SPH_FORM(kForceList, float, 2);
 SPH_FORM(kForceList, float, 3);
 SPH_FORM(kForceLanes, float, 2);
 SPH_FORM(kForceLanes, float, 3);
+SPH_FORM(kForceLanes, double, 2);
+SPH_FORM(kForceLanes, double, 3);
 SPH_FORM(kForceWalk, double, 2);
 SPH_FORM(kForceWalk, double, 3);
 #undef SPH_FORM
@@ -26,11 +28,13 @@ void launch_force(const View &v, int precision, int kernel, int viscosity, int h
     if (precision != SPH_MIXED) {
         if (v.n_tile > 0)
             tile_force(v, kernel, (viscosity ? 1 : 0) | (heat ? 2 : 0), integrator, stage, mode, s);
-        if (v.n_walk > 0)
+        if (v.n_walk > 0 && walk_lanes<double>(v) > 1)
+            run(launch_force_t<kForceLanes, double, 2>, launch_force_t<kForceLanes, double, 3>);
+        else if (v.n_walk > 0)
             run(launch_force_t<kForceWalk, double, 2>, launch_force_t<kForceWalk, double, 3>);
     } else if (v.vl_on) {
         run(launch_force_t<kForceList, float, 2>, launch_force_t<kForceList, float, 3>);
-    } else if (walk_lanes(v) > 1) {
+    } else if (walk_lanes<float>(v) > 1) {
         run(launch_force_t<kForceLanes, float, 2>, launch_force_t<kForceLanes, float, 3>);
     } else {
         run(launch_force_t<kForceWalk, float, 2>, launch_force_t<kForceWalk, float, 3>);

@@ -211,19 +211,17 @@ __global__ void __launch_bounds__(256, 5) k_heat_vl(const __grid_constant__ View
     heat_one<float, D, K, ONE, true>(v, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// The cell windows of a small mixed-precision launch, LANES lanes per particle:
-// one thread per particle would leave most SMs without a warp (1,024
-// particles: eight warps of 32) and every lane with the window's whole chain.
-// The epilogue runs on the first lane of each particle.
-template <int D, int K, int LANES>
+// The cell windows of a small launch, LANES lanes per particle: one thread per
+// particle would leave most SMs without a warp (1,024 particles: 32 warps) and
+// every lane with the window's whole chain.
+template <typename R, int D, int K, int LANES>
 __global__ void __launch_bounds__(256) k_density_lanes(const __grid_constant__ View v, int stage) {
-    density_one<float, D, K, false, false, LANES>(
+    density_one<R, D, K, false, false, LANES>(
         v, stage, (blockIdx.x * blockDim.x + threadIdx.x) / LANES);
 }
-template <int D, int K, int LANES>
+template <typename R, int D, int K, int LANES>
 __global__ void __launch_bounds__(256) k_heat_lanes(const __grid_constant__ View v) {
-    heat_one<float, D, K, false, false, LANES>(v,
-                                               (blockIdx.x * blockDim.x + threadIdx.x) / LANES);
+    heat_one<R, D, K, false, false, LANES>(v, (blockIdx.x * blockDim.x + threadIdx.x) / LANES);
 }
 
 // The persistent form is instantiated for the mixed-precision passes only;
@@ -236,17 +234,13 @@ void density_launch(const View &v, int stage, int block, cudaStream_t s) {
             k_density_vl<D, K, ONE><<<(v.np + block - 1) / block, block, 0, s>>>(v, stage);
             return;
         }
-        const int lanes = walk_lanes(v);
-        if (lanes == 32) {
-            k_density_lanes<D, K, 32><<<lanes_grid<32>(v), lanes_block<32>, 0, s>>>(v, stage);
-            return;
-        }
-        if (lanes == 8) {
-            k_density_lanes<D, K, 8><<<lanes_grid<8>(v), lanes_block<8>, 0, s>>>(v, stage);
-            return;
-        }
     }
-    if (std::is_same<R, float>::value && v.persist) {
+    const int lanes = walk_lanes<R>(v);
+    if (lanes == 32)
+        k_density_lanes<R, D, K, 32><<<lanes_grid<32>(v), lanes_block<32>, 0, s>>>(v, stage);
+    else if (lanes == 8)
+        k_density_lanes<R, D, K, 8><<<lanes_grid<8>(v), lanes_block<8>, 0, s>>>(v, stage);
+    else if (std::is_same<R, float>::value && v.persist) {
         auto *fn = k_density<R, D, K, ONE, std::is_same<R, float>::value>;
         fn<<<pass_grid(v, fn, block), block, 0, s>>>(v, stage);
     } else {
@@ -261,17 +255,13 @@ void heat_launch(const View &v, int block, cudaStream_t s) {
             k_heat_vl<D, K, ONE><<<(v.np + block - 1) / block, block, 0, s>>>(v);
             return;
         }
-        const int lanes = walk_lanes(v);
-        if (lanes == 32) {
-            k_heat_lanes<D, K, 32><<<lanes_grid<32>(v), lanes_block<32>, 0, s>>>(v);
-            return;
-        }
-        if (lanes == 8) {
-            k_heat_lanes<D, K, 8><<<lanes_grid<8>(v), lanes_block<8>, 0, s>>>(v);
-            return;
-        }
     }
-    if (std::is_same<R, float>::value && v.persist) {
+    const int lanes = walk_lanes<R>(v);
+    if (lanes == 32)
+        k_heat_lanes<R, D, K, 32><<<lanes_grid<32>(v), lanes_block<32>, 0, s>>>(v);
+    else if (lanes == 8)
+        k_heat_lanes<R, D, K, 8><<<lanes_grid<8>(v), lanes_block<8>, 0, s>>>(v);
+    else if (std::is_same<R, float>::value && v.persist) {
         auto *fn = k_heat<R, D, K, ONE, std::is_same<R, float>::value>;
         fn<<<pass_grid(v, fn, block), block, 0, s>>>(v);
     } else {

@@ -263,13 +263,14 @@ __device__ __forceinline__ void for_pairs_lanes(const View &v, const SimDev &S,
 
 // Adds the G lanes' blocks of a sum in lane order, on every lane: the lanes in
 // mask as BAcc::flush would.
-template <int G> __device__ __forceinline__ void fold_lanes(BAcc<float> &a, unsigned mask) {
+template <int G, typename R>
+__device__ __forceinline__ void fold_lanes(BAcc<R> &a, unsigned mask) {
 #pragma unroll 8
     for (int c = 0; c < G; ++c) {
-        const float x = __shfl_sync(0xffffffffu, a.part, c, G);
+        const R x = __shfl_sync(0xffffffffu, a.part, c, G);
         if (mask & (1u << c)) a.total.add(x);
     }
-    a.part = 0.0f;
+    a.part = (R)0;
 }
 
 // Window offset k - 3 of a list entry's 3-bit field k, as an exact float:
@@ -387,13 +388,20 @@ template <typename F> inline int pass_grid(const View &v, F *kernel, int block) 
     return nb < cap ? nb : cap;
 }
 
-// Lanes per particle of the mixed-precision cell-window passes, by the
-// particles of the launch (the bits do not depend on it).  All pair passes of a
-// step, us, with 1 / 8 / 32 lanes: 2D 1,024 particles 340 / 111 / 73, 4,096 325 /
-// 108 / 107, 16,384 352 / 185 / 247, 32,761 350 / 259 / 432, 65,536 375 / 432 /
-// 816; 3D with heat flux 2,197 particles 2122 / 615 / 274, 8,000 2124 / 608 / 675,
-// 32,768 2354 / 1923 / 2505, 64,000 2377 / 3041 / 4484.
-inline int walk_lanes(const View &v) { return v.np <= 4096 ? 32 : (v.np <= 40960 ? 8 : 1); }
+// Lanes per particle of the cell-window passes, by the particles of the launch (the
+// bits do not depend on it).  All pair passes of a step, us, with 1 / 8 / 32 lanes, mixed
+// precision: 2D 1,024 particles 340 / 111 / 73, 4,096 325 / 108 / 107, 16,384 352 / 185 /
+// 247, 32,761 350 / 259 / 432, 65,536 375 / 432 / 816; 3D with heat flux 2,197 particles
+// 2122 / 615 / 274, 8,000 2124 / 608 / 675, 32,768 2354 / 1923 / 2505, 64,000 2377 / 3041 /
+// 4484.  In FP64, whose pipe fills sooner (the simulations that are too sparse for cell
+// tiles), a step: 2D at 0.25 particles per cell 1,024 221 / 112 / 76, 2,704 239 / 121 / 170,
+// 4,096 243 / 120 / 202, 10,000 244 / 288 / 435; at 1.56 665 / 251 / 130, 676 / 259 / 311,
+// 672 / 251 / 375, 700 / 622 / 793; 3D with heat flux at 0.27 512 particles 997 / 501 / 232,
+// 2,197 1136 / 532 / 683, 4,096 1041 / 519 / 1090, 15,625 1166 / 1920 / 3584.
+template <typename R> inline int walk_lanes(const View &v) {
+    constexpr bool f64 = sizeof(R) == 8;
+    return v.np <= (f64 ? 1536 : 4096) ? 32 : (v.np <= (f64 ? 4096 : 40960) ? 8 : 1);
+}
 // Threads per block, and blocks, of the passes with LANES lanes per particle.  Their
 // epilogues (FP64, an instruction of which costs the pipe the same for one lane of a
 // warp as for all) are done by the block's first threads, one per particle, from
