@@ -156,8 +156,8 @@ struct sph_engine {
     int graph_steps = 0;
     bool graph_launched = false;   // its event slots hold a launch's profile
     bool props_valid = false;
-    void *xbuf = nullptr;          // workspace of the pair export
-    size_t xbuf_size = 0;
+    void *xrows = nullptr, *xbuf = nullptr;   // workspaces of the pair export
+    size_t xrows_size = 0, xbuf_size = 0;
 };
 
 namespace {
@@ -1328,21 +1328,23 @@ int write_state_range(sph_engine *e, int off, int64_t n, const double *r, const 
     return SPH_OK;
 }
 
-// Room of `bytes` in the pair export's workspace, keeping its first `keep` bytes.
-// The engine keeps the workspace between calls up to kExportKeep bytes.
+// Room of `bytes` in a workspace of the pair export, which keeps nothing of what it
+// held: the old memory is given back before the new is asked for.  The engine keeps
+// the row starts, and the pairs' workspace between calls up to kExportKeep bytes.
 constexpr size_t kExportKeep = size_t(256) << 20;
-int export_room(sph_engine *e, size_t bytes, size_t keep = 0) {
-    if (bytes <= e->xbuf_size) return SPH_OK;
-    const size_t want = std::max(bytes, std::min(bytes + bytes / 4, kExportKeep));
+int export_room(void **buf, size_t *size, size_t bytes) {
+    if (bytes <= *size) return SPH_OK;
+    cudaFree(*buf);
+    *buf = nullptr;
+    *size = 0;
+    size_t want = std::max(bytes, std::min(bytes + bytes / 4, kExportKeep));
     char *p = nullptr;
-    TRY(dalloc(&p, want));
-    if (keep) {
-        CK(cudaMemcpyAsync(p, e->xbuf, keep, cudaMemcpyDeviceToDevice, e->stream));
-        CK(cudaStreamSynchronize(e->stream));
+    if (dalloc(&p, want) != SPH_OK) {
+        want = bytes;
+        TRY(dalloc(&p, want));
     }
-    cudaFree(e->xbuf);
-    e->xbuf = p;
-    e->xbuf_size = want;
+    *buf = p;
+    *size = want;
     return SPH_OK;
 }
 
@@ -1481,7 +1483,8 @@ void free_all(sph_engine *e) {
                     e->pk_vel[0], e->pk_vel[1], e->pk_f, e->pk_q, e->pk_fv, e->ue, e->rho, e->rho_l,
                     e->temp, e->pres, e->pco, e->rho0, e->pres0, e->pco0, e->udot, e->f0u,
                     e->acc_u, e->stage_buf, e->sims_d, e->t_scale, e->tsum_part, e->steps_d,
-                    e->pair_count, e->err, e->err_any, e->rebin_gate, e->restage_far, e->n_items, e->mass_mixed, e->xbuf,
+                    e->pair_count, e->err, e->err_any, e->rebin_gate, e->restage_far, e->n_items, e->mass_mixed,
+                    e->xrows, e->xbuf,
                     e->bin_count,
                     e->chunk_sim, e->chunk_start,
                     e->chunk_len, e->cell_xyz};
@@ -1962,8 +1965,8 @@ int sph_sim_export_pairs(sph_engine *e, int32_t id, int64_t cap, int64_t *iap, d
     const Sim &S = e->sims[id];
     View v = make_view(e);
     stage_view(e, v, 0);
-    TRY(export_room(e, sizeof(long long) * ((size_t)S.n + 1)));
-    long long *rows = (long long *)e->xbuf;
+    TRY(export_room(&e->xrows, &e->xrows_size, sizeof(long long) * ((size_t)S.n + 1)));
+    long long *rows = (long long *)e->xrows;
     CK(cudaMemsetAsync(rows, 0, sizeof(long long) * (S.n + 1), st));
     launch_pair_rows(v, e->precision, S.part_off, (int)S.n, rows, st);
     launch_scan64(rows, (int)S.n, st);
@@ -1976,8 +1979,7 @@ int sph_sim_export_pairs(sph_engine *e, int32_t id, int64_t cap, int64_t *iap, d
     // the pairs found, in no order, and with host arrays a device copy of each
     const bool host = mem == SPH_HOST;
     const size_t np = (size_t)total, d = (size_t)e->dim;
-    const size_t at_found = sizeof(long long) * ((size_t)S.n + 1);
-    size_t at = at_found + sizeof(int2) * np;
+    size_t at = sizeof(int2) * np;
     auto take = [&](const void *want, size_t bytes) {
         const size_t here = at;
         if (want && host) at += bytes;
@@ -1985,14 +1987,13 @@ int sph_sim_export_pairs(sph_engine *e, int32_t id, int64_t cap, int64_t *iap, d
     };
     const size_t at_iap = take(iap, 16 * np), at_drij = take(drij, 8 * np * d);
     const size_t at_rsq = take(rsq, 8 * np), at_dv = take(dv, 8 * np * d);
-    int status = export_room(e, at, at_found);
-    if (status != SPH_OK) return status;
+    TRY(export_room(&e->xbuf, &e->xbuf_size, at));
     char *x = (char *)e->xbuf;
     auto place = [&](void *want, size_t here) {
         return !want ? nullptr : (host ? (void *)(x + here) : want);
     };
-    launch_pair_write(v, e->precision, S.part_off, (int)S.n, (const long long *)x,
-                      (int2 *)(x + at_found), (long long *)place(iap, at_iap),
+    launch_pair_write(v, e->precision, S.part_off, (int)S.n, rows, (int2 *)x,
+                      (long long *)place(iap, at_iap),
                       (double *)place(drij, at_drij), (double *)place(rsq, at_rsq),
                       (double *)place(dv, at_dv), st);
     if (host) {
