@@ -58,10 +58,11 @@ __device__ __forceinline__ Splat splat_prepare(const SplatArgs &A, int i, double
     if (A.dim3 && dz > A.cutoff) s.w = 0;
     const double pi = 3.14159265358979323846;
     const double wgt = A.a[i] * A.m[i] / A.rho[i], h = A.h[i];
-    // a smoothing length that is not positive draws zeros (wgt 0)
+    // a smoothing length that is not positive draws zeros (wgt 0), and so does one too
+    // small for its powers, off the particle itself (0 times a finite norm)
+    const double norm = A.dim3 ? 105.0 / (pi * 16.0 * (h * h * h)) : 5.0 / (pi * h * h);
     s.inv_h = h > 0.0 ? 1.0 / h : 0.0;
-    s.coef = wgt * (h > 0.0 ? (A.dim3 ? 105.0 / (pi * 16.0 * (h * h * h)) : 5.0 / (pi * h * h))
-                            : 0.0);
+    s.coef = wgt * (h > 0.0 ? fmin(norm, 1e300) : 0.0);
     return s;
 }
 
