@@ -49,24 +49,6 @@ constexpr int kTileCap = 256;
 using TileSlot = unsigned char;
 constexpr int kTileThreads = 32 * kTileRounds;
 
-// 1/r from r and ih = 1/(2r) to about 2^-40.
-__device__ __forceinline__ double tile_inv(double r, double ih) {
-    const double e = fma(-ih, r, 0.5);
-    const double h2 = ih + ih;
-    return fma(h2 + h2, e, h2);
-}
-
-__device__ __forceinline__ double tile_div(double n, double d) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    double e = fma(-d, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-d, y, 1.0);
-    y = fma(y, e, y);
-    const double q = n * y;
-    return fma(fma(-d, q, n), y, q);
-}
-
 // max(x, 0) for a finite x, without the FP64 pipe
 __device__ __forceinline__ double tile_pos(double x) {
     return __double2hiint(x) < 0 ? 0.0 : x;
