@@ -326,6 +326,23 @@ def serve_window(njobs, time_limit, budget_gb, seed=5000, dist=None, schemes=(0,
     return replicas.merge_served(replicas.gather(rep, dist))
 
 
+def result_line(line, details=None):
+    """The one JSON line of a run as text.  What grows with the jobs or the steps of a
+    sub-workload (the served window's record of every job, 60 KB for 200 of them) is
+    no part of it and goes to the file `details`, if one is given."""
+    out, rest = {}, {}
+    for k, v in line.items():
+        if k == "workloads":
+            v = {name: {a: b for a, b in w.items() if a != "job_records"}
+                 for name, w in v.items()}
+            rest["job_records"] = line[k].get("serve", {}).get("job_records")
+        out[k] = v
+    if details:
+        with open(details, "w") as f:
+            json.dump(rest, f)
+    return json.dumps(out)
+
+
 def run_e2e(prm, r, v, m, u, steps, torch, stream, knobs=None):
     """Through the C ABI with host (pinned) buffers: every step copies the
     state in, advances one step and reads the state back (the timed arm's
@@ -513,6 +530,8 @@ def main():
     ap.add_argument("--serve-budget-gb", type=float, default=3.0,
                     help="HBM budget of the served workload's engines")
     ap.add_argument("--serve-seconds", type=float, default=60.0)
+    ap.add_argument("--details", default=None,
+                    help="a file for the served window's per-job records")
     ap.add_argument("--accuracy-steps", type=int, default=1000,
                     help="trajectory length of the mixed-vs-FP64 accuracy report (0: skip)")
     ap.add_argument("--rebin", type=int, default=1, choices=[0, 1],
@@ -716,7 +735,7 @@ def main():
         line["latency"] = {"p50_s": sv.get("latency_p50_s"), "p99_s": sv.get("latency_p99_s"),
                            "workload": "served Poisson window (see workloads.serve)"}
         line["workloads"] = extras
-    print(json.dumps(line))
+    print(result_line(line, args.details))
     if dist:
         dist.destroy_process_group()
     return 0
