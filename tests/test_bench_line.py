@@ -1,6 +1,9 @@
 """bench.py prints one line that a reader with a small buffer can take in: the served
 window's per-job records go to a file of their own."""
 import json
+import os
+import subprocess
+import sys
 
 import bench
 
@@ -27,3 +30,13 @@ def test_records_go_to_a_file(tmp_path):
     bench.result_line(line(5), str(path))
     assert [r["job"] for r in json.loads(path.read_text())["job_records"]] == list(range(5))
     bench.result_line({"metric": bench.METRIC, "value": 1.0}, str(path))
+
+
+def test_reference_arm_says_that_there_is_none():
+    """Nothing of this repository is timed in the reference's name."""
+    path = os.path.join(bench.ROOT, "bench.py")
+    res = subprocess.run([sys.executable, path, "--impl", "reference", "--steps", "2"],
+                         capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr
+    got = json.loads(res.stdout)
+    assert got["impl"] == "reference" and got["unavailable"] and "value" not in got
