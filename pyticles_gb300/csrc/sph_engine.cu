@@ -126,6 +126,7 @@ struct sph_engine {
     int n_cell_sims = 0;           // live simulations on the cell-window passes
     int n_tile_sims = 0;           // ... of these, on cell tiles
     int items_max = 0;             // most work items of the cell tiles
+    int lane_load[2] = {0, 0};     // of the live simulations
     int *n_items = nullptr;
     int *mass_mixed = nullptr;     // per simulation slot: masses differ
     bool cl_disabled = false;      // cluster lists did not fit: cell passes only
@@ -688,6 +689,7 @@ View make_view(const sph_engine *e) {
     v.item_cell = e->rank;
     v.item_round = e->cell_of;
     v.items_max = e->items_max;
+    for (int k = 0; k < 2; ++k) v.lane_load[k] = e->lane_load[k];
     v.persist = e->tune.persistent;
     v.dim = e->dim;
     v.sims = e->sims_d;
@@ -908,7 +910,11 @@ int relayout(sph_engine *e) {
     TRY(cluster_setup(e, sd));
     TRY(vl_setup(e));
     e->n_cell_sims = e->n_tile_sims = 0;
-    int64_t items = 0;
+    int64_t items = 0, load[2] = {0, 0};
+    for (const auto &S : e->sims)
+        for (int k = 0; k < 2 && S.active; ++k)
+            load[k] += lane_load(e->dim, S.win, S.n, k == 0 ? 8 : 32);
+    for (int k = 0; k < 2; ++k) e->lane_load[k] = (int)std::min<int64_t>(load[k], INT32_MAX);
     for (int s = 0; s < (int)e->sims.size(); ++s)
         if (e->sims[s].active && !sd[s].cl_on) {
             ++e->n_cell_sims;

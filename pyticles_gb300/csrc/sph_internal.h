@@ -128,6 +128,7 @@ struct View {
     // binning (in the sort scratch, free by then); at most items_max
     int *n_items, *item_cell, *item_round;
     int items_max;
+    int lane_load[2];       // see lane_load(): with 8 and with 32 lanes per particle
     int dim;
     SimDev *sims;
     // state A
@@ -203,6 +204,14 @@ struct View {
 };
 
 constexpr int kTileRounds = 4;   // rounds of a cell in one item: a warp each
+
+// The particles of a simulation that G lanes each would keep as busy: the lanes share
+// out the cells of a particle's window, and those beyond its number stay idle.
+inline int64_t lane_load(int dim, const int *win, int64_t n, int G) {
+    int64_t cells = 1;
+    for (int a = 0; a < dim; ++a) cells *= 2 * win[a] + 1;
+    return n * ((cells + G - 1) / G * G) / cells;
+}
 
 // Strided view of an n x 3 (SoA, stride 1) or n x dim (row-major, stride
 // dim) FP64 array: element (slot, axis a) is p[a][slot * stride].

@@ -153,6 +153,8 @@ extern "C" int sph_derivatives_noalloc(const sph_params *p, int32_t precision, i
     w.n_tile = sd.tile_on;
     w.n_walk = 1 - sd.tile_on;
     w.dim = dim;
+    for (int k = 0; k < 2; ++k)
+        w.lane_load[k] = (int)lane_load(dim, sd.win, n, k == 0 ? 8 : 32);
     w.sims = c.take<SimDev>(1);
     for (int a = 0; a < 3; ++a) {
         w.a_pos[a] = c.take<double>(N);

@@ -388,19 +388,30 @@ template <typename F> inline int pass_grid(const View &v, F *kernel, int block) 
     return nb < cap ? nb : cap;
 }
 
-// Lanes per particle of the cell-window passes, by the particles of the launch (the
-// bits do not depend on it).  All pair passes of a step, us, with 1 / 8 / 32 lanes, mixed
-// precision: 2D 1,024 particles 340 / 111 / 73, 4,096 325 / 108 / 107, 16,384 352 / 185 /
-// 247, 32,761 350 / 259 / 432, 65,536 375 / 432 / 816; 3D with heat flux 2,197 particles
-// 2122 / 615 / 274, 8,000 2124 / 608 / 675, 32,768 2354 / 1923 / 2505, 64,000 2377 / 3041 /
-// 4484.  In FP64, whose pipe fills sooner (the simulations that are too sparse for cell
-// tiles), a step: 2D at 0.25 particles per cell 1,024 221 / 112 / 76, 2,704 239 / 121 / 170,
-// 4,096 243 / 120 / 202, 10,000 244 / 288 / 435; at 1.56 665 / 251 / 130, 676 / 259 / 311,
-// 672 / 251 / 375, 700 / 622 / 793; 3D with heat flux at 0.27 512 particles 997 / 501 / 232,
-// 2,197 1136 / 532 / 683, 4,096 1041 / 519 / 1090, 15,625 1166 / 1920 / 3584.
+// Lanes per particle of the cell-window passes, by the launch (the bits do not depend
+// on it).  A small launch is bound by the latency of one thread's window, which lanes
+// share; a larger one pays for lanes without a cell and for the fold.  Step, us, with
+// 1 / 8 / 32 lanes, mixed precision at nine (2D) or 12 (3D, with heat flux) particles per
+// cell: 2D 1,024 particles 340 / 111 / 73, 4,096 325 / 108 / 107, 16,384 352 / 185 / 247,
+// 32,761 350 / 259 / 432, 65,536 375 / 432 / 816; 3D 2,197 2122 / 615 / 274, 8,000 2124 /
+// 608 / 675, 32,768 2354 / 1923 / 2505, 64,000 2377 / 3041 / 4484.  With fewer particles
+// in a cell the line is earlier: 2D at 0.25 28,900 115 / 106, 36,100 117 / 125, at 2.25 40,000
+// 197 / 168; 3D at 0.27 27,000 407 / 370, 39,304 424 / 529, at 1.33 27,000 577 / 458, 39,304
+// 596 / 676.  Windows of few cells (axes of a single cell) leave lanes idle, hence the
+// limits on lane_load: one cell, which has nothing to share, 40 x 1,000 particles in 3D 2408 /
+// 7515, 64 particles 90 / 95 / 106; five cells 3D 20,000 1672 / 1627, 40,000 1739 / 2555,
+// 2D 20,000 200 / 167; 25 cells 3D 20,250 1592 / 1200, 36,000 1639 / 1757.
+// FP64, whose pipe fills sooner (simulations too sparse for cell tiles): 2D at 0.25 1,024
+// 221 / 112 / 76, 2,704 239 / 121 / 170, 4,096 243 / 120 / 202, 10,000 244 / 288 / 435; at
+// 1.56 665 / 251 / 130, 676 / 259 / 311, 672 / 251 / 375, 700 / 622 / 793; 3D at 0.27 512
+// 997 / 501 / 232, 2,197 1136 / 532 / 683, 4,096 1041 / 519 / 1090, 15,625 1166 / 1920 / 3584.
 template <typename R> inline int walk_lanes(const View &v) {
-    constexpr bool f64 = sizeof(R) == 8;
-    return v.np <= (f64 ? 1536 : 4096) ? 32 : (v.np <= (f64 ? 4096 : 40960) ? 8 : 1);
+    if (v.lane_load[0] >= 8LL * v.np) return 1;   // windows of one cell
+    if (sizeof(R) == 8) return v.np <= 1536 ? 32 : (v.np <= 4096 ? 8 : 1);
+    const bool dense = v.np >= (v.dim == 2 ? 2LL : 4LL) * v.ncells;
+    if (v.np <= 4096 && v.lane_load[1] <= 65536) return 32;
+    if (v.np <= (dense ? 40960 : 28672) && v.lane_load[0] <= (v.dim == 2 ? 52428 : 41943)) return 8;
+    return 1;
 }
 // Threads per block, and blocks, of the passes with LANES lanes per particle.  Their
 // epilogues (FP64, an instruction of which costs the pipe the same for one lane of a
