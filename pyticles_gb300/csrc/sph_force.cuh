@@ -213,7 +213,11 @@ __device__ __forceinline__ void force_finish(const View &v, const SimDev &S, int
 // simulation, whose constants come from the kernel parameters.
 // Register caps by resident blocks of 256 threads; force of a step, us: a single
 // simulation in 2D (199k particles) 324 / 337 / 294 at 4 / 5 / 6 blocks, in 3D (205k)
-// 2178 / 2248 / 2649 at 3 / 4 / 5; 24 simulations in 2D 524 / 531 / 514 at 3 / 4 / 5.
+// 2248 / 2649 at 4 / 5.  3D at 3 blocks is 3% faster at 205k, whose last wave it fills,
+// and slower elsewhere; whole step at 3 / 4: 46,656 particles 1684 / 1727, 125,000 2668 /
+// 2344, 205,379 3444 / 3497, 343,000 5336 / 5309, 729,000 10154 / 9751, 1,331,000 18098 /
+// 17391.  Several in 2D at 5 / 4: 24 of 16,900 944 / 935, with a cutoff of 1.5 491 / 456,
+// 3 of 90,000 684 / 669.
 // LIST: the pair lists (tuning.pair_scheme 2) instead of the cell windows.
 // LANES: lanes per particle (for_pairs_lanes; the same bits).
 template <typename R, int D, int K, int VH, bool ONE, bool LIST = false, int LANES = 1>
@@ -368,7 +372,7 @@ __device__ __forceinline__ void force_one(const View &v, int stage, int mode, in
 // One thread per particle; PERSIST: the resident blocks of pass_grid walk
 // the particles grid-stride (the same per-particle work, the same bits).
 template <typename R, int D, int K, int VH, bool ONE, bool PERSIST>
-__global__ void __launch_bounds__(256, ONE ? (D == 2 ? 6 : 3) : (D == 2 ? 5 : 4)) k_force(const __grid_constant__ View v, int stage,
+__global__ void __launch_bounds__(256, ONE && D == 2 ? 6 : 4) k_force(const __grid_constant__ View v, int stage,
                                                   int mode, int integ) {
     if constexpr (PERSIST) {
         for (int base = blockIdx.x * blockDim.x; base < v.np; base += gridDim.x * blockDim.x)

@@ -16,7 +16,10 @@ namespace sph {
 // Register caps by resident blocks of 256 threads.  A single simulation (its
 // constants are kernel parameters) runs best at 6 (40 registers): density of
 // a step, us, at 5 / 6 / 7 blocks 252 / 229 / 233 in 2D (199k particles) and 1625 /
-// 1429 / 1446 in 3D (205k); several at 4 (391 us against 418 at 5).
+// 1429 / 1446 in 3D (205k); several at 4 (391 us against 418 at 5).  3D at other sizes,
+// whole step at 5 / 6: 97,336 particles 2041 / 2063, 157,464 2952 / 2977, 729,000 9822 /
+// 9751, 1,331,000 17553 / 17391; at 0.6 particles per cell 125,000 593 / 641, 729,000
+// 2725 / 2793.
 // LIST: the pair lists (tuning.pair_scheme 2) instead of the cell windows.
 // LANES: lanes per particle (for_pairs_lanes; the same bits).
 template <typename R, int D, int K, bool ONE, bool LIST = false, int LANES = 1>
