@@ -26,7 +26,8 @@ __device__ __forceinline__ double min_image(double d, double L) {
 }
 
 struct SplatArgs {
-    int n, cols, nx, ny, dim3, per;   // per: particles of a warp
+    int n, cols, nx, ny, dim3;
+    int per, own;   // particles of a warp; most pixels that a lane draws by itself
     const double *r, *m, *rho, *a, *h, *x, *y;
     double z, xmin, xmax, ymin, ymax, cutoff;
     double *Z;
@@ -91,6 +92,15 @@ struct SplatQueue {
     unsigned char k[64];   // the particle, as the lane that prepared it
 };
 
+// One pixel of a particle at squared distance rsq.
+__device__ __forceinline__ void splat_pixel(const SplatArgs &A, int xx, int yy, double rsq,
+                                            double coef, double inv_h) {
+    // Lucy: q (1 + 3 s/h) (1 - s/h)^3
+    double ih, t = fma(-sph::tile_sqrt(rsq, &ih), inv_h, 1.0);
+    if (__double2hiint(t) < 0) t = 0.0;
+    atomicAdd(&A.Z[(size_t)xx * A.ny + yy], coef * (t * t * t) * fma(-3.0, t, 4.0));
+}
+
 // Draws one found pixel per lane (the first `n` of the queue).
 __device__ __forceinline__ void splat_draw(const SplatArgs &A, const SplatQueue &q, int n,
                                            const Splat &mine) {
@@ -98,11 +108,23 @@ __device__ __forceinline__ void splat_draw(const SplatArgs &A, const SplatQueue 
     const double coef = __shfl_sync(0xffffffffu, mine.coef, k);
     const double inv_h = __shfl_sync(0xffffffffu, mine.inv_h, k);
     if (lane >= n) return;
-    // Lucy: q (1 + 3 s/h) (1 - s/h)^3
-    double ih, t = fma(-sph::tile_sqrt(q.rsq[lane], &ih), inv_h, 1.0);
-    if (__double2hiint(t) < 0) t = 0.0;
-    const int2 px = q.px[lane];
-    atomicAdd(&A.Z[(size_t)px.x * A.ny + px.y], coef * (t * t * t) * fma(-3.0, t, 4.0));
+    splat_pixel(A, q.px[lane].x, q.px[lane].y, q.rsq[lane], coef, inv_h);
+}
+
+// The pixels of the lane's own particle.
+__device__ __forceinline__ void splat_own(const SplatArgs &A, const Splat &s, double c2) {
+    for (int col = 0; col < s.w; ++col) {
+        const int xx = wrap_once(s.xa + col, A.nx);
+        if (xx < 0 || xx >= A.nx) continue;
+        const double dx = fast_image(s.rx - A.x[xx], A.xmax);
+        for (int row = 0; row < s.hgt; ++row) {
+            const int yy = wrap_once(s.ya + row, A.ny);
+            if (yy < 0 || yy >= A.ny) continue;
+            const double dy = fast_image(A.y[yy] - s.ry, A.ymax);
+            const double rsq = dx * dx + fma(dy, dy, s.dz2);
+            if (fast_less(rsq, c2)) splat_pixel(A, xx, yy, rsq, s.coef, s.inv_h);
+        }
+    }
 }
 
 // A warp per `per` particles: each lane prepares one (the divisions of a
@@ -113,6 +135,12 @@ __device__ __forceinline__ void splat_draw(const SplatArgs &A, const SplatQueue 
 // kernel, has no idle lanes.  One thread per particle took 1.29 ms for 100,172
 // particles on 635 x 633 pixels (94 pixels each), a lane per pixel without the
 // queue 0.74 ms, this form 0.47 ms.
+// Boxes of few pixels leave that form's lanes idle one particle after the other: a warp
+// of such boxes alone draws them with a lane per particle, up to 36 pixels a box, fewer
+// in proportion where a warp has fewer than 32 particles.  Queue / lane, us, 2D on 600^2
+// pixels: 1,000,000 particles of 1.4 pixels 1055 / 227, of 13 1200 / 652, of 36 1698 /
+// 1126, of 52 1961 / 2121; 20,000 (16 to a warp) of 13 63 / 59, of 36 77 / 87; 3,000 (two)
+// of 6 36 / 40.
 __global__ void __launch_bounds__(128) k_splat(const SplatArgs A) {
     __shared__ SplatQueue queues[4];
     SplatQueue &q = queues[threadIdx.x >> 5];
@@ -122,6 +150,10 @@ __global__ void __launch_bounds__(128) k_splat(const SplatArgs A) {
     const double res = A.x[1] - A.x[0], c2 = A.cutoff * A.cutoff;
     const int count = min(A.per, A.n - first);
     const Splat mine = splat_prepare(A, min(first + lane, A.n - 1), res);
+    if (__all_sync(0xffffffffu, mine.w <= A.own && mine.hgt <= A.own && mine.w * mine.hgt <= A.own)) {
+        if (lane < count) splat_own(A, mine, c2);
+        return;
+    }
     int queued = 0;
     for (int k = 0; k < count; ++k) {
         const int w = __shfl_sync(0xffffffffu, mine.w, k);
@@ -242,7 +274,7 @@ extern "C" int sph_splash_map(int32_t mode, int64_t n, const double *r, int32_t 
         const int sms = sph::device_sms();
         const int per = (int)std::min<int64_t>(32, std::max<int64_t>(1, n / (8 * sms)));
         const SplatArgs A = {(int)n,    r_cols,    nx,        ny,        mode == 3 ? 1 : 0,
-                             per,       dr,        dm,        drho,      da,
+                             per,       36 * per / 32, dr,        dm,        drho,      da,
                              dh,        dx,        dy,        z,         bounds[0],
                              bounds[1], bounds[2], bounds[3], cutoff,    dZ};
         const int64_t warps = (n + per - 1) / per;
