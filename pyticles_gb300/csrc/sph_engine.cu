@@ -400,9 +400,13 @@ bool tile_scheme(const sph_engine *e, const Sim &S) {
 // Lanes per particle (log2) of the cell tiles: 32 for a small simulation, which
 // spreads it over more warps, eight otherwise.  Density + force of a step, us,
 // 32 / 16 / 8 lanes: 2D 1,024 particles 94 / 107 / 112, 4,096 230 / 214 / 180;
-// 3D 2,197 particles 571 / 711 / 920, 8,000 1934 / 1691 / 1704.
-constexpr int64_t kTileSmall = 3072;
-int tile_lanes(int64_t n) { return n <= kTileSmall ? 5 : 3; }
+// 3D 2,197 particles 571 / 711 / 920, 8,000 1934 / 1691 / 1704.  Eight as well for a
+// handful of particles, which have no candidates for 32 lanes; step of 1,000 of them,
+// 32 / 8 lanes / window walk: 9 particles each 262 / 115 / 129, 25 602 / 359 / 455, 36 1022 /
+// 695 / 634, 64 2172 / 1366 / 2103; of one, 9 particles 47 / 47 / 107, 36 52 / 76 / 319, 64 60
+// / 91 / 536.
+constexpr int64_t kTileFew = 64, kTileSmall = 3072;
+int tile_lanes(int64_t n) { return n > kTileFew && n <= kTileSmall ? 5 : 3; }
 // Most work items of a simulation.
 int64_t tile_items(int64_t n, int ncells) {
     const int per = kTileRounds * (32 >> tile_lanes(n));
