@@ -261,7 +261,9 @@ typedef struct sph_tuning {
                                  walk the flattened particle table grid-
                                  stride: one persistent launch per pass over
                                  all simulations.  Each particle's sums are
-                                 the same either way (same bits)           */
+                                 the same either way (same bits).  Small
+                                 launches, which take several lanes per
+                                 particle, and FP64 ones ignore it         */
     double list_skin;         /* pair_scheme 2: the lists' skin as a fraction of
                                  the cutoff (0.01 .. 0.5; default 0.025); at
                                  least 32 dt vmax is used                     */

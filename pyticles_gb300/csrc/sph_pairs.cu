@@ -507,7 +507,9 @@ void launch_pair_write(const View &v, int precision, int sim_off, int n,
 #undef SPH_EXPORT
 
 // Exclusive scan of n + 1 int64 entries in place (export path only): one block,
-// eight entries a thread and two barriers per 8,192.
+// eight entries a thread and one barrier per 8,192.  The sums of a round lie in one of
+// two buffers: a warp that writes a buffer again, two rounds later, has passed the
+// barrier in between, which every reader of its old content reached after reading.
 constexpr int kScan64Per = 8;
 __global__ void __launch_bounds__(1024) k_scan64(long long *data, int n) {
     __shared__ long long warp_sum[2][32];

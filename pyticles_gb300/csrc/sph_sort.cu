@@ -222,7 +222,9 @@ static void launch_cellsort(const View &v, int ncells, cudaStream_t s) {
 // and block barriers is shorter than the one through six kernels.  Binning of a step,
 // six kernels / one, us: 2D 256 particles 25.2 / 15.9, 1k 25.4 / 18.6, 2k 26.3 / 22.6,
 // 4k 26.5 / 29.3; 3D 1.7k 27.7 / 25.5, 3.4k 28.7 / 35.1; 512 particles in few cells
-// 167 / 25.  The step of the 1k fluid: 81.8 -> 75.6 us.
+// 167 / 25.  The step of the 1k fluid: 81.8 -> 75.6 us.  By cells, a step of sparse
+// particles, six / one: 16 particles 256 cells 43.4 / 35.2, 8,190 45.8 / 41.3; 512 particles
+// 1,024 51.4 / 42.7, 8,190 50.5 / 46.3; 2,000 particles 1,024 56.5 / 54.2, 6,300 53.2 / 51.6.
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallParticles = 2048, kSmallCells = 8192;
 constexpr int kSmallPer = kSmallParticles / kSmallThreads;

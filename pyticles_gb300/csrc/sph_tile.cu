@@ -586,36 +586,35 @@ __device__ __forceinline__ void tile_round(const View &v, const SimDev &S, Mem &
             unsigned far = in & ~near;
             int drop = 0;   // candidates of the guard band that are no pairs
             // the accepted candidates, dealt out evenly through the queue
-const int own = __popc(near) | (__popc(far) << 16);
-int incl = own;
-for (int o = 1; o < G; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o, G);
-    if (l >= o) incl += y;
-}
-const int tot = __shfl_sync(0xffffffffu, incl, G - 1, G);
-int pn = (incl - own) & 0xffff, pf = kTileCap - 1 - ((incl - own) >> 16);
-TileSlot *qu = queue->q[slot];
-__syncwarp();   // the last sub-tile's readers are done
-while (near) {
-    const int q = top_bit(near);
-    near ^= 1u << q;
-    qu[pn++] = (TileSlot)(top - (q << lg));
-}
-while (far) {
-    const int q = top_bit(far);
-    far ^= 1u << q;
-    qu[pf--] = (TileSlot)(top - (q << lg));
-}
-__syncwarp();
-const int nn = tot & 0xffff, nf = tot >> 16;
-if (l == 0) npairs += nn + nf;
-for (int t = l; t < nn; t += G)
-    tile_pair<true, D>(v, S, mem, qu[t], i, pi, thr_lo, drop, pass);
-if (Pass::kFar)
-    for (int t = l; t < nf; t += G)
-        tile_pair<false, D>(v, S, mem, qu[kTileCap - 1 - t], i, pi, thr_lo,
-                           drop, pass);
-__syncwarp();
+            const int own = __popc(near) | (__popc(far) << 16);
+            int incl = own;
+            for (int o = 1; o < G; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o, G);
+                if (l >= o) incl += y;
+            }
+            const int tot = __shfl_sync(0xffffffffu, incl, G - 1, G);
+            int pn = (incl - own) & 0xffff, pf = kTileCap - 1 - ((incl - own) >> 16);
+            TileSlot *qu = queue->q[slot];
+            __syncwarp();   // the last sub-tile's readers are done
+            while (near) {
+                const int q = top_bit(near);
+                near ^= 1u << q;
+                qu[pn++] = (TileSlot)(top - (q << lg));
+            }
+            while (far) {
+                const int q = top_bit(far);
+                far ^= 1u << q;
+                qu[pf--] = (TileSlot)(top - (q << lg));
+            }
+            __syncwarp();
+            const int nn = tot & 0xffff, nf = tot >> 16;
+            if (l == 0) npairs += nn + nf;
+            for (int t = l; t < nn; t += G)
+                tile_pair<true, D>(v, S, mem, qu[t], i, pi, thr_lo, drop, pass);
+            if (Pass::kFar)
+                for (int t = l; t < nf; t += G)
+                    tile_pair<false, D>(v, S, mem, qu[kTileCap - 1 - t], i, pi, thr_lo, drop, pass);
+            __syncwarp();
             npairs -= drop;
         }
     } while (more);
@@ -697,9 +696,7 @@ __global__ void __launch_bounds__(kTileThreads, 4)
 template <typename Pass, typename F, typename... Args>
 void tile_launch(F *kernel, const View &v, cudaStream_t s, Args... args) {
     constexpr size_t smem = sizeof(TileSmem<Pass>);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+    static_assert(smem <= 48 * 1024, "a block's shared memory without an opt-in");
     const int grid = std::max(1, std::min(v.items_max, 64 * device_sms()));
     kernel<<<grid, kTileThreads, smem, s>>>(v, args...);
 }
