@@ -5,9 +5,9 @@
 // One thread per particle that walks its own window (for_pairs) spends them on
 // every candidate's test and runs its loop bodies at half of its lanes; here
 //
-//  * candidates are tested in packed FP32, two per instruction, 1e-6 too wide
-//    (inside the guard band the bodies ask the exact FP64 test), so that FP64
-//    work begins with the pair;
+//  * candidates are tested in packed FP32, two per instruction, as much too wide as
+//    its rounding asks (fast_margin, short_support2; inside the guard band the bodies
+//    ask the exact FP64 test), so that FP64 work begins with the pair;
 //  * accepted candidates go through a queue in shared memory, pairs within the
 //    short support from its front and the others from its back, so that the
 //    bodies run with all lanes busy and the two kinds never diverge;
@@ -32,9 +32,8 @@
 // after a block barrier, one thread per particle of the item.
 //
 // Measured, density / force pass in us, for_pairs -> tiles: 2D 1,024 particles
-// 300 / 458 -> 21 / 25, 65,535 particles 887 / 1403 -> 352 / 497 (FP64 pipe 75-78%
-// busy, 78 FP64 warp instructions per particle in the density pass); 3D 2,197
-// particles 1988 / 2666 -> 110 / 175.
+// 300 / 458 -> 21 / 25, 65,536 particles 887 / 1403 -> 352 / 495 (FP64 pipe 78 / 81%
+// busy); 3D 2,197 particles 1988 / 2666 -> 110 / 172 (76 / 79%).
 #include <algorithm>
 
 #include "sph_force.cuh"
