@@ -45,3 +45,30 @@ def test_a_kept_state_is_the_start_of_the_next_step(dim, precision, scheme, inte
     _, ref, _, _ = oracle.advance(prm, r2, v2, m2, u1, 1)
     # the step's change of velocity is its mean rate times dt
     assert rel_l2(got - v2, ref - v2) < (1e-5 if precision == "mixed" else 1e-9)
+
+
+@pytest.mark.parametrize("precision,scheme", [("mixed", 0), ("mixed", 2), ("fp64", 0)])
+def test_one_simulation_of_a_batch(precision, scheme):
+    """The others go on from where they were."""
+    sims = []
+    for k, side in enumerate((24, 32, 40)):
+        prm, r, v, m, T0 = workloads.config_2d(side, 1010 + k, viscosity=True)
+        sims.append((prm, r, v, m, oracle.initial_energy(prm, r, v, m, T0)))
+    rng = np.random.default_rng(13)
+    with Engine(sims[0][0], precision, max_particles=sum(len(s[1]) for s in sims),
+                max_sims=3) as e:
+        ids = [e.add(*s) for s in sims]
+        e.set_tuning(pair_scheme=scheme, rebin=1, steps_per_graph=1)
+        e.advance(1)
+        states = [e.get_state(i) for i in ids]
+        bins = e.rebin_count()
+        r, v, u = states[1]
+        states[1] = (r + 1e-3 * rng.uniform(-1, 1, r.shape), v + rng.normal(0, 1, v.shape), u)
+        e.set_state(ids[1], states[1][0], states[1][1], sims[1][3], u)
+        e.advance(1)
+        e.sync()
+        assert e.rebin_count() == bins
+        got = [e.get_state(i)[1] for i in ids]
+    for s, (r, v, u), g in zip(sims, states, got):
+        _, ref, _, _ = oracle.advance(s[0], r, v, s[3], u, 1)
+        assert rel_l2(g - v, ref - v) < (1e-5 if precision == "mixed" else 1e-9)
